@@ -324,71 +324,168 @@ GB_DEV bool child_fails( const IntArgs<R> &a, const R (&u)[5], bool prim )
    return bad;
 }
 
-// Interpolate_Iterate for the five conserved hydro variables (INTERP_MASK: each parent on its own)
+// the attempts after the first of Interpolate_Iterate for one parent (primitive variables, then the
+// reduced coefficients), and the store of what they end with; the rare path, out of line so that the
+// first attempt keeps its children in registers.  (i, j, k): the parent in the coarse cells cb
 template <int SCH, typename R>
-__global__ void interp_iterate_kernel( const __grid_constant__ IntArgs<R> a )
+__device__ __noinline__ void iterate_parent( const IntArgs<R> &a, const R *cb, size_t c3, int i, int j, int k, R *fo )
 {
-   const int nx = a.crange[0], nxy = a.crange[0]*a.crange[1], ncell = nxy*a.crange[2];
-   const size_t c3 = (size_t)a.csize[0]*a.csize[1]*a.csize[2], f3 = (size_t)a.fsize[0]*a.fsize[1]*a.fsize[2];
+   const size_t fx = a.fsize[0], fxy = (size_t)a.fsize[0]*a.fsize[1], f3 = fxy*a.fsize[2];
    const int mono_iter = a.mono_max_iter;
    const int max_iter = a.int_prim ? mono_iter + 1 : mono_iter;
-   for (long long t = blockIdx.x*(long long)blockDim.x + threadIdx.x; t < (long long)ncell*a.nbatch;
-        t += (long long)gridDim.x*blockDim.x)
+   R f[5][2][2][2];
+   bool prim = false, ok = false;
+   R coeff = a.mono_coeff;
+   for (int it = 1; it <= max_iter && !ok; it++)
    {
-      const int c = (int)( t % ncell ), b = (int)( t / ncell );
-      const int ii = c % nx, jj = ( c / nx ) % a.crange[1], kk = c / nxy;
-      const int i = a.cstart[0] + ii, j = a.cstart[1] + jj, k = a.cstart[2] + kk;
-      const R *cb = a.cdata + (size_t)b*5*c3;
-      R f[5][2][2][2];
-      bool prim = false, ok = false;
-      R coeff = a.mono_coeff;
-      for (int it = 0; it <= max_iter && !ok; it++)
+      if ( it == 1 && a.int_prim ) prim = true;
+      else coeff = rmax( rsub( coeff, rdiv( a.mono_coeff, (R)mono_iter ) ), R(0) );
+#     pragma unroll 1
+      for (int v=0; v<5; v++) children<SCH>( a, cb, c3, v, i, j, k, prim, coeff, f[v] );
+      ok = true;
+#     pragma unroll 1
+      for (int q=0; q<8; q++)
       {
-         if ( it == 1 && a.int_prim ) prim = true;
-         else if ( it >= 1 ) coeff = rmax( rsub( coeff, rdiv( a.mono_coeff, (R)mono_iter ) ), R(0) );
-         // one variable at a time (the children of all five are kept for the checks)
-#        pragma unroll 1
-         for (int v=0; v<5; v++) children<SCH>( a, cb, c3, v, i, j, k, prim, coeff, f[v] );
-         ok = true;
+         R u[5];
 #        pragma unroll
-         for (int q=0; q<8; q++)
-         {
-            R u[5];
-#           pragma unroll
-            for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
-            ok &= !child_fails( a, u, prim );
-         }
+         for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+         ok &= !child_fails( a, u, prim );
       }
-      if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
-      R *fb = a.fdata + (size_t)b*5*f3;
+   }
+   if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
+#  pragma unroll 1
+   for (int q=0; q<8; q++)
+   {
+      const int dz = q >> 2, dy = ( q >> 1 ) & 1, dx = q & 1;
+      R u[5];
+#     pragma unroll
+      for (int v=0; v<5; v++) u[v] = f[v][dz][dy][dx];
+      if ( prim )
+      {
+         // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
+         const R d = u[0];
+         u[1] = rmul( d, u[1] );  u[2] = rmul( d, u[2] );  u[3] = rmul( d, u[3] );
+         const R eint = rmul( u[4], a.inv_gm1 );
+         u[4] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( u[1], u[1] ), rmul( u[2], u[2] ) ), rmul( u[3], u[3] ) ) ), d ), eint );
+      }
+#     pragma unroll
+      for (int v=0; v<5; v++) fo[v*f3 + dz*fxy + dy*fx + dx] = u[v];
+   }
+}
+
+// Interpolate_Iterate for the five conserved hydro variables (INTERP_MASK: each parent on its own).
+// One CTA takes `depth` planes of parents of one region, so that the 27 (125) coarse cells around
+// each parent come from shared memory (STAGED; a region whose planes are too wide for that is read
+// from global memory).  The children of the five variables stay in registers: with a run-time loop
+// over the variables they went through local memory.  Bound by the issue of the 19 one-dimensional
+// operators of a parent's variable, each of rounded multiplications and selects.  With the assembly
+// below, 342 windows of 20^3, FP32: 217 -> 97 us (the bytes of both alone: 27 us).
+constexpr int INT_THREADS = 256;
+
+// CTAs per SM: 342 regions of 12^3 cells, with the window assembly, us: FP32 1: 137, 2: 111, 3: 97, 4: 103
+// (6 of 128 threads: 103); FP64 (229 regions) 1: 149, 2: 118, 3: 120, 4: 123
+template <typename R> constexpr int int_ctas() { return sizeof(R) == 4 ? 3 : 2; }
+
+template <int SCH, typename R, bool STAGED>
+__global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_kernel( const __grid_constant__ IntArgs<R> a, int depth, int nslab )
+{
+   constexpr int G = int_ghost( SCH );
+   extern __shared__ __align__(16) unsigned char int_smem[];
+   const int b = blockIdx.x / nslab, k0 = ( blockIdx.x % nslab )*depth;
+   const int nk = ( a.crange[2] - k0 < depth ) ? a.crange[2] - k0 : depth;
+   const int nx = a.crange[0], nxy = a.crange[0]*a.crange[1], cxy = a.csize[0]*a.csize[1];
+   const size_t fx = a.fsize[0], fxy = (size_t)a.fsize[0]*a.fsize[1], f3 = fxy*a.fsize[2];
+   const size_t c3 = (size_t)cxy*a.csize[2];
+   const R *cb = a.cdata + (size_t)b*5*c3;
+   const int n = ( nk + 2*G )*cxy;                                   // coarse cells staged per variable
+   const int kbase = STAGED ? a.cstart[2] + k0 - G : 0;              // their first plane
+   const size_t cs = STAGED ? (size_t)n : c3;
+   const R *src = STAGED ? (const R*)int_smem : cb;
+   if constexpr ( STAGED )
+   {
+      R *s_c = (R*)int_smem;
+      const R *g = cb + (size_t)kbase*cxy;
+      // 16-byte loads where the array and whole planes are 16-byte aligned
+      constexpr int V = 16/sizeof(R);
+      if ( cxy % V == 0 && ( (uintptr_t)a.cdata & 15u ) == 0 )
+      {
+         for (int e = threadIdx.x; e < n/V; e += INT_THREADS)
+#           pragma unroll
+            for (int v=0; v<5; v++) ( (uint4*)( s_c + v*n ) )[e] = ( (const uint4*)( g + v*c3 ) )[e];
+      }
+      else
+         for (int e = threadIdx.x; e < n; e += INT_THREADS)
+#           pragma unroll
+            for (int v=0; v<5; v++) s_c[v*n + e] = g[v*c3 + e];
+      __syncthreads();
+   }
+   for (int c = threadIdx.x; c < nxy*nk; c += INT_THREADS)
+   {
+      const int ii = c % nx, jj = ( c / nx ) % a.crange[1], kk = k0 + c / nxy;
+      const int i = a.cstart[0] + ii, j = a.cstart[1] + jj, k = a.cstart[2] + kk - kbase;
+      // Interpolate_Iterate stores from the origin of the fine region
+      R *fo = a.fdata + (size_t)b*5*f3 + (size_t)( 2*kk )*fxy + (size_t)( 2*jj )*fx + 2*ii;
+      R f[5][2][2][2];
+#     pragma unroll
+      for (int v=0; v<5; v++)
+      {
+         children<SCH>( a, src, cs, v, i, j, k, false, a.mono_coeff, f[v] );
+         asm volatile( "" ::: "memory" );      // one variable's stencil live at a time
+      }
+      bool ok = true;
 #     pragma unroll
       for (int q=0; q<8; q++)
       {
-         const int fz = q >> 2, fy = ( q >> 1 ) & 1, fx = q & 1;
          R u[5];
 #        pragma unroll
-         for (int v=0; v<5; v++) u[v] = f[v][fz][fy][fx];
-         if ( prim )
-         {
-            // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
-            const R d = u[0];
-            u[1] = rmul( d, u[1] );  u[2] = rmul( d, u[2] );  u[3] = rmul( d, u[3] );
-            const R eint = rmul( u[4], a.inv_gm1 );
-            u[4] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( u[1], u[1] ), rmul( u[2], u[2] ) ), rmul( u[3], u[3] ) ) ), d ), eint );
-         }
-         const size_t o = (size_t)( a.fstart[2] + 2*kk + fz )*a.fsize[0]*a.fsize[1] + ( a.fstart[1] + 2*jj + fy )*a.fsize[0] +
-                          ( a.fstart[0] + 2*ii + fx );
-#        pragma unroll
-         for (int v=0; v<5; v++) fb[(size_t)v*f3 + o] = u[v];
+         for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+         ok &= !child_fails( a, u, false );
       }
+      if ( !ok ) { iterate_parent<SCH>( a, src, cs, i, j, k, fo );  continue; }
+#     pragma unroll
+      for (int v=0; v<5; v++)
+#        pragma unroll
+         for (int q=0; q<8; q++) fo[v*f3 + ( q >> 2 )*fxy + ( ( q >> 1 ) & 1 )*fx + ( q & 1 )] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
    }
+}
+
+// planes of parents per CTA and their shared memory: half the parents' planes, fewer where those need
+// more than 48 KB (four CTAs share an SM), one at least; 0 bytes where even that needs over 200 KB
+template <typename R>
+int interp_depth( int scheme, const IntArgs<R> &a, size_t *smem )
+{
+   const int G = int_ghost( scheme );
+   const size_t plane = (size_t)5*a.csize[0]*a.csize[1]*sizeof(R);
+   int depth = ( a.crange[2] + 1 )/2;
+   while ( depth > 1 && ( depth + 2*G )*plane > 48*1024 ) depth--;
+   *smem = ( depth + 2*G )*plane;
+   if ( *smem > 200*1024 ) *smem = 0;
+   return depth;
+}
+
+template <int SCH, typename R>
+cudaError_t iterate_launch( const IntArgs<R> &a, cudaStream_t st )
+{
+   size_t smem = 0;
+   const int depth = interp_depth( SCH, a, &smem ), nslab = ( a.crange[2] + depth - 1 )/depth;
+   const long long grid = (long long)nslab*a.nbatch;
+   if ( grid > 0x7fffffffLL ) return cudaErrorInvalidValue;
+   if ( smem == 0 ) interp_iterate_kernel<SCH,R,false><<< (unsigned)grid, INT_THREADS, 0, st >>>( a, depth, nslab );
+   else
+   {
+      const cudaError_t e = ( smem <= 48*1024 ) ? cudaSuccess
+         : cudaFuncSetAttribute( interp_iterate_kernel<SCH,R,true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200*1024 );
+      if ( e != cudaSuccess ) return e;
+      interp_iterate_kernel<SCH,R,true><<< (unsigned)grid, INT_THREADS, smem, st >>>( a, depth, nslab );
+   }
+   return cudaGetLastError();
 }
 
 template <typename R>
 cudaError_t interp_launch( int scheme, bool iterate, const IntArgs<R> &a, cudaStream_t st )
 {
    const long long ncell = (long long)a.crange[0]*a.crange[1]*a.crange[2];
-   const long long items = ncell*a.nbatch*( iterate ? 1 : a.ncomp );
+   const long long items = ncell*a.nbatch*a.ncomp;
    constexpr int B = 128;
    long long g = ( items + B - 1 )/B;
    int dev = 0, nsm = 148;
@@ -397,8 +494,8 @@ cudaError_t interp_launch( int scheme, bool iterate, const IntArgs<R> &a, cudaSt
    if ( g > 32LL*nsm ) g = 32LL*nsm;
    if ( g < 1 ) return cudaSuccess;
 #  define GB_INT_CASE( S ) \
-   case S: if ( iterate ) interp_iterate_kernel<S,R><<< (unsigned)g, B, 0, st >>>( a ); \
-           else           interp_kernel<S,R><<< (unsigned)g, B, 0, st >>>( a ); break;
+   case S: if ( iterate ) return iterate_launch<S,R>( a, st ); \
+           interp_kernel<S,R><<< (unsigned)g, B, 0, st >>>( a );  break;
    switch ( scheme )
    {
       GB_INT_CASE( INT_MINMOD3D )
@@ -439,36 +536,79 @@ int interp_run( const gb_interp_params *p, const void *cdata, void *fdata, int n
 // ---- window assembly of the ghost-zone fill ------------------------------------------------------
 // Prepare_PatchData (src/Main/Prepare_PatchData.cpp) fills each side of a patch group's window from
 // the patch groups of the same level where they exist and by interpolation from the coarser level
-// where they do not (InterpolateGhostZone).  Here: one thread per window cell and variable; the side
-// of the cell picks its source -- the patch group's own interior, the interior of the same-level patch
-// group nbr[p][s], or the coarse-interpolated window cint[p] (gb_interpolate_device over the window).
-template <typename R>
-__global__ void assemble_windows_kernel( const R *fine, const int *nbr, const R *cint, R *win, int npg, int ncomp,
-                                         int nxt )
+// where they do not (InterpolateGhostZone).  Here the side of a cell picks its source -- the patch
+// group's own interior, the interior of the same-level patch group nbr[p][s], or the
+// coarse-interpolated window cint[p] (gb_interpolate_device over the window).
+//
+// One CTA fills the window of one variable of one patch group; the 27 sources are resolved once into
+// shared memory.  A thread writes four consecutive cells with 16-byte stores (VEC: a window is a
+// whole number of them, since its width is even; an array that is not 16-byte aligned takes scalar
+// stores).  NXT: the width, a constant for the usual ones, so that the index arithmetic divides by
+// constants.
+constexpr int ASM_THREADS = 256;
+
+template <typename R, int NXT, bool VEC>
+__global__ void __launch_bounds__( ASM_THREADS ) assemble_windows_kernel( const R *fine, const int *nbr, const R *cint, R *win,
+                                                                          int npg, int ncomp, int nxt_any )
 {
-   const int g = ( nxt - PS2 )/2, n3 = nxt*nxt*nxt;
-   const long long total = (long long)npg*ncomp*n3;
-   for (long long t = blockIdx.x*(long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x*blockDim.x)
+   const int nxt = NXT ? NXT : nxt_any;
+   const int g = ( nxt - PS2 )/2, n2 = nxt*nxt, n3 = nxt*n2;
+   constexpr int PS3 = PS2*PS2*PS2;
+   constexpr long long FROM_CINT = -1, NO_SOURCE = -2;
+   __shared__ long long s_src[27];      // first element of the source interior, or one of the above
+   for (long long pv = blockIdx.x; pv < (long long)npg*ncomp; pv += gridDim.x)
    {
-      const int c = (int)( t % n3 );
-      const long long pv = t / n3;
       const int v = (int)( pv % ncomp ), p = (int)( pv / ncomp );
-      const int i = c % nxt, j = ( c / nxt ) % nxt, k = c / ( nxt*nxt );
-      int x = i - g, y = j - g, z = k - g;
-      const int dx = ( x < 0 ) ? -1 : ( x >= PS2 ), dy = ( y < 0 ) ? -1 : ( y >= PS2 ), dz = ( z < 0 ) ? -1 : ( z >= PS2 );
-      int src = p;
-      if ( dx | dy | dz )
+      __syncthreads();
+      if ( threadIdx.x < 27 )
       {
-         src = nbr[p*27 + ( dz + 1 )*9 + ( dy + 1 )*3 + ( dx + 1 )];
-         x -= PS2*dx;  y -= PS2*dy;  z -= PS2*dz;
+         const int src = ( threadIdx.x == 13 ) ? p : nbr[(size_t)p*27 + threadIdx.x];
+         // NO_SOURCE: not a patch group of the batch, or a coarse side without an interpolated window
+         s_src[threadIdx.x] = ( src >= npg ) ? NO_SOURCE : ( src >= 0 ) ? ( (long long)src*ncomp + v )*PS3
+                                                                         : ( cint != nullptr ) ? FROM_CINT : NO_SOURCE;
       }
-      R val;
-      if ( src >= npg ) val = R(NAN);    // not a patch group of the batch
-      else if ( src >= 0 ) val = fine[( (size_t)src*ncomp + v )*PS2*PS2*PS2 + ( z*PS2 + y )*PS2 + x];
-      else if ( cint )     val = cint[( (size_t)p*ncomp + v )*n3 + c];
-      else                 val = R(NAN);  // a coarse side without an interpolated window
-      win[( (size_t)p*ncomp + v )*n3 + c] = val;
+      __syncthreads();
+      const R *ci = cint + (size_t)pv*n3;
+      R *wo = win + (size_t)pv*n3;
+      for (int c0 = 4*threadIdx.x; c0 < n3; c0 += 4*ASM_THREADS)
+      {
+         R val[4];
+#        pragma unroll
+         for (int q=0; q<4; q++)
+         {
+            const int c = c0 + q;
+            const int k = c / n2, r = c - k*n2, j = r / nxt, i = r - j*nxt;
+            const int x = i - g, y = j - g, z = k - g;
+            const int dx = ( x < 0 ) ? -1 : ( x >= PS2 ), dy = ( y < 0 ) ? -1 : ( y >= PS2 ), dz = ( z < 0 ) ? -1 : ( z >= PS2 );
+            const long long src = s_src[( dz + 1 )*9 + ( dy + 1 )*3 + ( dx + 1 )];
+            val[q] = ( src >= 0 ) ? fine[src + ( ( z - PS2*dz )*PS2 + ( y - PS2*dy ) )*PS2 + ( x - PS2*dx )]
+                                  : ( src == FROM_CINT ) ? ci[c] : R(NAN);
+         }
+         if constexpr ( !VEC )
+         {
+#           pragma unroll
+            for (int q=0; q<4; q++) wo[c0 + q] = val[q];
+         }
+         else if constexpr ( sizeof(R) == 4 ) *(float4*)( wo + c0 ) = make_float4( val[0], val[1], val[2], val[3] );
+         else { ( (double2*)( wo + c0 ) )[0] = make_double2( val[0], val[1] );  ( (double2*)( wo + c0 ) )[1] = make_double2( val[2], val[3] ); }
+      }
    }
+}
+
+template <typename R>
+int assemble_launch( const void *fine, const int *nbr, const void *cint, void *win, int npg, int ncomp, int nxt, cudaStream_t st )
+{
+   const long long items = (long long)npg*ncomp;
+   const unsigned grid = (unsigned)( ( items < 0x7fffffffLL ) ? items : 0x7fffffffLL );
+   const bool vec = ( (uintptr_t)win & 15u ) == 0;
+#  define GB_ASM( N, V ) assemble_windows_kernel<R,N,V><<< grid, ASM_THREADS, 0, st >>>( (const R*)fine, nbr, (const R*)cint, (R*)win, npg, ncomp, nxt )
+   if      ( !vec )      GB_ASM( 0, false );
+   else if ( nxt == 20 ) GB_ASM( 20, true );
+   else if ( nxt == 22 ) GB_ASM( 22, true );
+   else if ( nxt == 24 ) GB_ASM( 24, true );
+   else                  GB_ASM( 0, true );
+#  undef GB_ASM
+   return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
 }
 
 } // namespace
@@ -520,19 +660,7 @@ int gb_assemble_windows_device( const void *fine, const int *nbr, const void *ci
    if ( precision != GB_PREC_FP32 && precision != GB_PREC_FP64 ) return GB_E_INVALID;
    if ( npg == 0 ) return GB_OK;
    if ( fine == nullptr || nbr == nullptr || windows == nullptr ) return GB_E_INVALID;
-   const long long total = (long long)npg*ncomp*nxt*nxt*nxt;
-   constexpr int B = 256;
-   int dev = 0, nsm = 148;
-   cudaGetDevice( &dev );
-   cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
-   long long g = ( total + B - 1 )/B;
-   if ( g > 16LL*nsm ) g = 16LL*nsm;
    cudaStream_t st = (cudaStream_t)stream;
-   if ( precision == GB_PREC_FP64 )
-      assemble_windows_kernel<double><<< (unsigned)g, B, 0, st >>>( (const double*)fine, nbr, (const double*)cint,
-                                                                    (double*)windows, npg, ncomp, nxt );
-   else
-      assemble_windows_kernel<float><<< (unsigned)g, B, 0, st >>>( (const float*)fine, nbr, (const float*)cint,
-                                                                   (float*)windows, npg, ncomp, nxt );
-   return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
+   return ( precision == GB_PREC_FP64 ) ? assemble_launch<double>( fine, nbr, cint, windows, npg, ncomp, nxt, st )
+                                        : assemble_launch<float> ( fine, nbr, cint, windows, npg, ncomp, nxt, st );
 }
