@@ -12,45 +12,14 @@
 // reconstruction (traced with the entropy wave, :555-562), the Riemann solvers (upwinded with the
 // mass flux) and the transverse correction, floored by PassiveFloor, and the full step ends with the
 // dual-energy fix of Hydro_FullStepUpdate (CPU_Shared_FullStepUpdate.cpp:144-201).
-#include <cstring>
-#include <type_traits>
-#include "../../include/gamer_b200_fluid.h"
-#include "hydro_physics.cuh"
+#include "ctu_hydro.cuh"
 
 namespace gb {
 
-namespace hctu {
-constexpr int NX  = 20;                // FLU_NXT
-constexpr int NX3 = NX*NX*NX;
-constexpr int NF  = 18;                // N_FC_VAR = N_HF_FLUX = N_FL_FLUX
-constexpr int NF3 = NF*NF*NF;
-// input sizes of the reconstruction LR: PLM FLU_NXT 20 (LR_GHOST_SIZE 1, FLU_GHOST_SIZE 2), PPM
-// FLU_NXT 22 (2, 3) (include/Macro.h:643-665); the face-state, flux and output grids are the same
-template <int LR> struct G {
-   static constexpr int NX  = ( LR == LR_PPM ) ? 22 : 20;   // FLU_NXT
-   static constexpr int NX3 = NX*NX*NX;
-   static constexpr int LRG = ( LR == LR_PPM ) ? 2 : 1;     // LR_GHOST_SIZE
-   static constexpr int FLG = LRG + 1;                       // FLU_GHOST_SIZE
-};
-
-GB_DEV int idx3( int i, int j, int k, int ni, int nj ) { return ( k*nj + j )*ni + i; }
-
-template <typename R>
-struct Args {
-   const R *in;      // [npg][NC][20^3]
-   R *out;           // [npg][NC][16^3]
-   R *flux;          // [npg][9][NC][16^2]  (nullptr: not stored)
-   char *de;         // [npg][16^3] dual-energy status (NC = 6 or 8; nullptr: not stored)
-   R *pri;           // scratch [npg][NC][20^3]
-   R *fcv;           // scratch [npg][6][NC][18^3]
-   R *fcf;           // scratch [npg][3][NC][18^3]
-   int npg, limiter;
-   int nnorm;        // NormPassive: number of listed passive scalars (0 = off)
-   int norm_idx[4];  // NormIdx (passive indices, no repeats)
-   R coeff, dt, dh;
-   Phys<R> ph;
-};
-}
+// the plane-streaming kernel (ctu_fused.cuh), one instantiation unit per policy
+int ctu_fused_fp32 ( const gb_fluid_config &cfg, const void *in, void *out, void *flux, int npg, const gb_fluid_params *prm, int *status, cudaStream_t st );
+int ctu_fused_mixed( const gb_fluid_config &cfg, const void *in, void *out, void *flux, int npg, const gb_fluid_params *prm, int *status, cudaStream_t st );
+int ctu_fused_fp64 ( const gb_fluid_config &cfg, const void *in, void *out, void *flux, int npg, const gb_fluid_params *prm, int *status, cudaStream_t st );
 
 // items of one patch group per grid.z index (blockIdx.z = patch group of the chunk), 32-bit indices
 #define HCTU_PG_LOOP( r, per ) \
@@ -83,240 +52,6 @@ __global__ void hctu_con2pri( const __grid_constant__ hctu::Args<R> a )
    }
 }
 
-// ---- PLM + characteristic tracing along D (CPU_Shared_DataReconstruction.cpp:376-560, hydro) ----
-// Hydro_GetEigenSystem (:1611-1892, no MHD): eigenvalues v_d - a, v_d (x3), v_d + a; the left and
-// right eigenvectors in the rotated frame (rho, v_n, v_t1, v_t2, P) do not depend on the direction.
-// RS: the HLL solvers trace with all waves (:454-477, HLL_INCLUDE_ALL_WAVES); Roe and the exact
-// solver trace each face from the reference state of the fastest wave toward it (:513-553)
-// CH: CHAR_RECONSTRUCTION, the PLM slopes limited in the characteristic variables of the cell
-// LR_PPM: PPM face values (:704-1135, the limited slopes of the cell and its two neighbours, the
-// parabola and its monotonicity constraint) and the tracing of the parabola (:1136-1290): each
-// wave's correction over its domain of dependence adds the curvature term dfc6 = 6 (cc - (fL+fR)/2)
-template <int D, int RS, int NC, int CH, int LR, typename R>
-GB_DEV void hctu_recon_dir( const hctu::Args<R> &a, const R *pri, const R *cc, int c, R (&fcon)[2][NC] )
-{
-   using namespace hctu;
-   typedef Dir<D> M;
-   constexpr int NX = G<LR>::NX, NX3 = G<LR>::NX3;
-   const int dcc[3] = { 1, NX, NX*NX };
-   const R rho = cc[0], irho = R(1)/rho;
-   const R a2 = a.ph.gamma*cc[4]/rho, as = gsqrt( a2 ), ia = R(1)/as, ia2 = ia*ia;
-   R LE[5][5], RE[5][5];
-#  pragma unroll
-   for (int r=0; r<5; r++)
-#     pragma unroll
-      for (int q=0; q<5; q++) { LE[r][q] = R(0);  RE[r][q] = R(0); }
-   LE[0][1] = -R(0.5)*rho*ia;  LE[0][4] = R(0.5)*ia2;
-   LE[1][0] = R(1);            LE[1][4] = -ia2;
-   LE[2][2] = R(1);            LE[3][3] = R(1);
-   LE[4][1] = -LE[0][1];       LE[4][4] = LE[0][4];
-   RE[0][0] = R(1);  RE[0][1] = -as*irho;  RE[0][4] = a2;
-   RE[1][0] = R(1);
-   RE[2][2] = R(1);  RE[3][3] = R(1);
-   RE[4][0] = R(1);  RE[4][1] = -RE[0][1];  RE[4][4] = a2;
-   const R vn = cc[M::n];
-   const R ev[5] = { vn - as, vn, vn, vn, vn + as };
-   R fl[NC], fr[NC];
-   if constexpr ( LR == LR_PPM )
-   {
-      // the slopes of the cells c-1, c, c+1 (limited in primitive or characteristic variables)
-      R sl[NC], sc[NC], sr[NC];
-      if constexpr ( CH )
-      {
-         R ll[NC], cl[NC], cr[NC], rr[NC];
-#        pragma unroll
-         for (int v=0; v<NC; v++)
-         {
-            const R *q = pri + v*NX3 + c;
-            ll[v] = q[-2*dcc[D]];  cl[v] = q[-dcc[D]];  cr[v] = q[dcc[D]];  rr[v] = q[2*dcc[D]];
-         }
-         ppm_char_slopes<D,NC>( a.ph, ll, cl, cc, cr, rr, a.limiter, a.coeff, sl, sc, sr );
-      }
-      else
-      {
-#        pragma unroll
-         for (int v=0; v<NC; v++)
-         {
-            const R *q = pri + v*NX3 + c;
-            sl[v] = limit_slope( q[-2*dcc[D]], q[-dcc[D]], q[0],         a.limiter, a.coeff );
-            sc[v] = limit_slope( q[-dcc[D]],   q[0],       q[dcc[D]],    a.limiter, a.coeff );
-            sr[v] = limit_slope( q[0],         q[dcc[D]],  q[2*dcc[D]],  a.limiter, a.coeff );
-         }
-      }
-#     pragma unroll
-      for (int v=0; v<NC; v++)
-         ppm_faces( pri[v*NX3 + c - dcc[D]], cc[v], pri[v*NX3 + c + dcc[D]], sl[v], sc[v], sr[v], a.limiter, fl[v], fr[v] );
-   }
-   else if constexpr ( CH )
-   {
-      R cl[NC], cr[NC];
-#     pragma unroll
-      for (int v=0; v<NC; v++) { cl[v] = pri[v*NX3 + c - dcc[D]];  cr[v] = pri[v*NX3 + c + dcc[D]]; }
-      plm_faces_char<D,NC>( a.ph, cl, cc, cr, a.limiter, a.coeff, fl, fr );
-   }
-   else
-   {
-#     pragma unroll
-      for (int v=0; v<NC; v++)
-      {
-         const R l = pri[v*NX3 + c - dcc[D]], r = pri[v*NX3 + c + dcc[D]];
-         plm_faces( l, cc[v], r, a.limiter, a.coeff, true, fl[v], fr[v] );
-      }
-   }
-   const R dt_dh2 = R(0.5)*a.dt/a.dh;
-   const int wv[5] = { 0, M::n, M::t1, M::t2, 4 };
-   R dfc[5];
-#  pragma unroll
-   for (int q=0; q<5; q++) dfc[q] = fr[wv[q]] - fl[wv[q]];
-   if constexpr ( LR == LR_PPM )
-   {
-      // PPM (:1145-1257): dfc6 = 6 (cc - (fL + fR)/2) in the rotated frame
-      R dfc6[5];
-#     pragma unroll
-      for (int q=0; q<5; q++) dfc6[q] = R(6)*( cc[wv[q]] - R(0.5)*( fl[wv[q]] + fr[wv[q]] ) );
-      R corl[5], corr[5];
-      if constexpr ( RS == RS_HLLC || RS == RS_HLLE )
-      {
-         // all waves toward both faces (HLL_INCLUDE_ALL_WAVES)
-#        pragma unroll
-         for (int q=0; q<5; q++) { corl[q] = R(0);  corr[q] = R(0); }
-#        pragma unroll
-         for (int m=0; m<5; m++)
-         {
-            const R cC = -dt_dh2*ev[m], cD = R(-4.0/3.0)*( cC*cC );
-            R cfl = R(0), cfr = R(0);
-#           pragma unroll
-            for (int q=0; q<5; q++)
-            {
-               cfl += LE[m][q]*( cC*( dfc[q] + dfc6[q] ) + cD*dfc6[q] );
-               cfr += LE[m][q]*( cC*( dfc[q] - dfc6[q] ) + cD*dfc6[q] );
-            }
-#           pragma unroll
-            for (int q=0; q<5; q++) { corl[q] = corl[q] + mul_rn( cfl, RE[m][q] );  corr[q] = corr[q] + mul_rn( cfr, RE[m][q] ); }
-         }
-      }
-      else
-      {
-         // Roe / exact: the reference states of the fastest waves, then the waves toward each face
-         const R cl0 = -dt_dh2*gmin( ev[0], R(0) ), cr0 = -dt_dh2*gmax( ev[4], R(0) );
-#        pragma unroll
-         for (int q=0; q<5; q++)
-         {
-            corl[q] = cl0*( dfc[q] + ( R(1) - R(4.0/3.0)*cl0 )*dfc6[q] );
-            corr[q] = cr0*( dfc[q] - ( R(1) + R(4.0/3.0)*cr0 )*dfc6[q] );
-         }
-#        pragma unroll
-         for (int m=0; m<5; m++)
-         {
-            if ( ev[m] <= R(0) )
-            {
-               const R cC = dt_dh2*( ev[0] - ev[m] ), cD = R(4.0/3.0)*dt_dh2*cC*( ev[0] + ev[m] );
-               R cf = R(0);
-#              pragma unroll
-               for (int q=0; q<5; q++) cf += LE[m][q]*( cC*( dfc[q] + dfc6[q] ) + cD*dfc6[q] );
-#              pragma unroll
-               for (int q=0; q<5; q++) corl[q] = corl[q] + mul_rn( cf, RE[m][q] );
-            }
-            if ( ev[m] >= R(0) )
-            {
-               const R cA = dt_dh2*( ev[4] - ev[m] ), cB = R(4.0/3.0)*dt_dh2*cA*( ev[4] + ev[m] );
-               R cf = R(0);
-#              pragma unroll
-               for (int q=0; q<5; q++) cf += LE[m][q]*( cA*( dfc[q] - dfc6[q] ) + cB*dfc6[q] );
-#              pragma unroll
-               for (int q=0; q<5; q++) corr[q] = corr[q] + mul_rn( cf, RE[m][q] );
-            }
-         }
-      }
-      // passive scalars with the entropy wave, the parabola integrated over its domain (:1262-1273)
-      if constexpr ( NC > 5 )
-      {
-         const R cl = -dt_dh2*gmin( ev[1], R(0) ), cr = -dt_dh2*gmax( ev[1], R(0) );
-#        pragma unroll
-         for (int v=5; v<NC; v++)
-         {
-            const R dv = fr[v] - fl[v], dv6 = R(6)*( cc[v] - R(0.5)*( fl[v] + fr[v] ) );
-            fl[v] += cl*( dv + ( R(1) - R(4.0/3.0)*cl )*dv6 );
-            fr[v] += cr*( dv - ( R(1) + R(4.0/3.0)*cr )*dv6 );
-         }
-      }
-#     pragma unroll
-      for (int q=0; q<5; q++) { fl[wv[q]] += corl[q];  fr[wv[q]] += corr[q]; }
-   }
-   else if constexpr ( RS == RS_HLLC || RS == RS_HLLE )
-   {
-      // HLL solvers: corrections from all waves, the same on both faces (HLL_INCLUDE_ALL_WAVES)
-      R corr[5];
-#     pragma unroll
-      for (int q=0; q<5; q++) corr[q] = R(0);
-#     pragma unroll
-      for (int m=0; m<5; m++)
-      {
-         R cf = R(0);
-#        pragma unroll
-         for (int q=0; q<5; q++) cf += LE[m][q]*dfc[q];
-         cf *= -dt_dh2*ev[m];
-         // uncontracted, as the reference's CPU build: sums that cancel do so exactly
-#        pragma unroll
-         for (int q=0; q<5; q++) corr[q] = corr[q] + mul_rn( cf, RE[m][q] );
-      }
-#     pragma unroll
-      for (int q=0; q<5; q++) { fl[wv[q]] += corr[q];  fr[wv[q]] += corr[q]; }
-   }
-   else
-   {
-      // Roe / exact: each face from the reference state of the fastest wave moving toward it, then
-      // the waves moving toward the face relative to it
-      const R cl0 = -dt_dh2*gmin( ev[0], R(0) ), cr0 = -dt_dh2*gmax( ev[4], R(0) );
-      R corl[5], corr[5];
-#     pragma unroll
-      for (int q=0; q<5; q++) { corl[q] = mul_rn( cl0, dfc[q] );  corr[q] = mul_rn( cr0, dfc[q] ); }
-#     pragma unroll
-      for (int m=0; m<5; m++)
-      {
-         if ( ev[m] <= R(0) )
-         {
-            R cf = R(0);
-#           pragma unroll
-            for (int q=0; q<5; q++) cf += LE[m][q]*dfc[q];
-            cf *= dt_dh2*( ev[0] - ev[m] );
-#           pragma unroll
-            for (int q=0; q<5; q++) corl[q] = corl[q] + mul_rn( cf, RE[m][q] );
-         }
-         if ( ev[m] >= R(0) )
-         {
-            R cf = R(0);
-#           pragma unroll
-            for (int q=0; q<5; q++) cf += LE[m][q]*dfc[q];
-            cf *= dt_dh2*( ev[4] - ev[m] );
-#           pragma unroll
-            for (int q=0; q<5; q++) corr[q] = corr[q] + mul_rn( cf, RE[m][q] );
-         }
-      }
-#     pragma unroll
-      for (int q=0; q<5; q++) { fl[wv[q]] += corl[q];  fr[wv[q]] += corr[q]; }
-   }
-   // passive scalars travel with the flow: the entropy wave only (:555-562; PPM above)
-   if constexpr ( NC > 5 && LR == LR_PLM )
-   {
-      const R cl = -dt_dh2*gmin( ev[1], R(0) ), cr = -dt_dh2*gmax( ev[1], R(0) );
-#     pragma unroll
-      for (int v=5; v<NC; v++)
-      {
-         const R dv = fr[v] - fl[v];
-         fl[v] += cl*dv;
-         fr[v] += cr*dv;
-      }
-   }
-   fl[0] = gmax( fl[0], a.ph.min_dens );  fr[0] = gmax( fr[0], a.ph.min_dens );
-   fl[4] = check_floor( fl[4], a.ph.min_pres );  fr[4] = check_floor( fr[4], a.ph.min_pres );
-#  pragma unroll
-   for (int v=5; v<NC; v++)
-      if ( a.ph.pfloor & ( 1u << v ) ) { fl[v] = gmax( fl[v], Lim<R>::tiny() );  fr[v] = gmax( fr[v], Lim<R>::tiny() ); }
-   pri2con<NC>( a.ph, fl, fcon[0] );
-   pri2con<NC>( a.ph, fr, fcon[1] );
-}
-
 template <typename R, int P, int RS, int NC, int CH, int LR>
 __global__ void __launch_bounds__( 256, ( sizeof(R) == 8 ) ? 1 : 4 ) hctu_recon( const __grid_constant__ hctu::Args<R> a )
 {
@@ -331,9 +66,13 @@ __global__ void __launch_bounds__( 256, ( sizeof(R) == 8 ) ? 1 : 4 ) hctu_recon(
       R cc[NC], fcon[2][NC];
 #     pragma unroll
       for (int v=0; v<NC; v++) cc[v] = pri[v*NX3 + c];
-      if      ( d == 0 ) hctu_recon_dir<0,RS,NC,CH,LR>( a, pri, cc, c, fcon );
-      else if ( d == 1 ) hctu_recon_dir<1,RS,NC,CH,LR>( a, pri, cc, c, fcon );
-      else               hctu_recon_dir<2,RS,NC,CH,LR>( a, pri, cc, c, fcon );
+      const R dt_dh2 = R(0.5)*a.dt/a.dh, *q = pri + c;
+      R fl[NC], fr[NC];
+      if      ( d == 0 ) hctu_faces<0,RS,NC,CH,LR>( a.ph, a.limiter, a.coeff, true, dt_dh2, q - 2, q - 1, cc, q + 1, q + 2, NX3, fl, fr );
+      else if ( d == 1 ) hctu_faces<1,RS,NC,CH,LR>( a.ph, a.limiter, a.coeff, true, dt_dh2, q - 2*NX, q - NX, cc, q + NX, q + 2*NX, NX3, fl, fr );
+      else               hctu_faces<2,RS,NC,CH,LR>( a.ph, a.limiter, a.coeff, true, dt_dh2, q - 2*NX*NX, q - NX*NX, cc, q + NX*NX, q + 2*NX*NX, NX3, fl, fr );
+      pri2con<NC>( a.ph, fl, fcon[0] );
+      pri2con<NC>( a.ph, fr, fcon[1] );
       R *fcv = a.fcv + (size_t)pg*6*NC*NF3;
 #     pragma unroll
       for (int q=0; q<2; q++)
@@ -494,6 +233,28 @@ __global__ void hctu_update( const __grid_constant__ hctu::Args<R> a )
    }
 }
 
+// Whether a call of npg patch groups runs through the plane-streaming kernel: five variables, limiting
+// in primitive variables, and HLLC, HLLE or Roe (PPM: not with Roe, 2.13 against 2.00 ms at 1000
+// patch groups; not in FP64, whose planes need 266 KB of shared memory).
+// It takes one time T per wave of patch groups (one or two CTAs per SM), 19 dependent steps long,
+// while the separate kernels spread any number over the whole GPU and take a time t per patch group:
+// the line lies at npg = T/t per wave.  Measured on B200, us: FP32 PLM HLLC T 121, t 1.21 (100 patch
+// groups: 121 / 129, 40: 121 / 59, 4096: 2030 / 4364); PPM T 176, t 1.77; FP64 T 211, t 2.08 (1000:
+// 1461 / 2079).  Mixed T 234, t 1.13 on a flow where every cell takes the double recovery; Roe T 285, t
+// 1.23 (1000: 1141 / 1232).
+bool ctu_hydro_fused( const gb_fluid_config &cfg, int npg )
+{
+   const bool ppm = ( cfg.lr_scheme == GB_LR_PPM ), fp64 = ( cfg.precision == GB_PREC_FP64 );
+   if ( cfg.dual_energy != GB_DE_NONE || cfg.npassive_user != 0 || cfg.char_reconstruction ) return false;
+   if ( cfg.rsolver == GB_RSOLVER_EXACT || ( ppm && ( fp64 || cfg.rsolver == GB_RSOLVER_ROE ) ) ) return false;
+   int dev = 0, nsm = 148;
+   cudaGetDevice( &dev );
+   cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
+   const int slots = nsm*( ( ppm || fp64 ) ? 1 : 2 ), waves = ( npg + slots - 1 )/slots;
+   const int line = ( !fp64 && ( cfg.precision == GB_PREC_MIXED || cfg.rsolver != GB_RSOLVER_HLLC ) ) ? 235 : 100;
+   return npg > 0 && npg >= line*waves;
+}
+
 namespace {
 
 size_t hctu_scratch_per_pg( size_t rsz, int nc, int lr )
@@ -524,34 +285,10 @@ int hctu_solve_t( const gb_fluid_config &cfg, const void *in, void *out, void *f
       const int n = ( npg - p0 < chunk ) ? npg - p0 : chunk;
       char *w = (char*)scratch;
       auto take = [&]( size_t elems ) { R *r = (R*)w;  w += ( elems*sizeof(R) + 255 ) & ~(size_t)255;  return r; };
-      Args<R> a;
-      memset( &a, 0, sizeof(a) );
-      a.in   = (const R*)in  + (size_t)p0*NC*NX3;
-      a.out  = (R*)out + (size_t)p0*NC*PS2*PS2*PS2;
-      a.flux = ( prm->store_flux && flux ) ? (R*)flux + (size_t)p0*9*NC*PS2*PS2 : nullptr;
-      a.de   = ( NC > 5 && de ) ? de + (size_t)p0*PS2*PS2*PS2 : nullptr;
+      Args<R> a = hctu_args<R,NC,LR>( cfg, in, out, flux, de, p0, n, prm );
       a.pri  = take( (size_t)n*NC*NX3 );
       a.fcv  = take( (size_t)n*6*NC*NF3 );
       a.fcf  = take( (size_t)n*3*NC*NF3 );
-      a.npg  = n;
-      a.limiter = prm->lr_limiter;
-      a.coeff = (R)prm->minmod_coeff;
-      a.dt = (R)prm->dt;  a.dh = (R)prm->dh;
-      a.ph.gamma = (R)cfg.gamma;  a.ph.gm1 = (R)( cfg.gamma - 1.0 );  a.ph.inv_gm1 = (R)( 1.0/( cfg.gamma - 1.0 ) );
-      a.ph.min_dens = (R)prm->min_dens;  a.ph.min_pres = (R)prm->min_pres;  a.ph.min_eint = (R)prm->min_eint;
-      a.ph.de_switch = (R)prm->dual_energy_switch;
-      a.ph.jeans = prm->jeans_min_pres;  a.ph.jeans_coeff = (R)prm->jeans_min_pres_coeff;
-      a.ph.pfloor = 0u;
-      for (int v=5; v<NC; v++) if ( prm->passive_floor & ( 1LL << v ) ) a.ph.pfloor |= 1u << v;
-      // FracPassive (mass fractions in the reconstruction) and NormPassive of the user scalars
-      a.ph.frac_mask = 0u;
-      if ( prm->frac_passive ) for (int k=0; k<prm->nfrac; k++) a.ph.frac_mask |= 1u << prm->frac_idx[k];
-      a.nnorm = 0;
-      if ( prm->norm_passive )
-      {
-         a.nnorm = prm->nnorm;
-         for (int k=0; k<prm->nnorm && k<4; k++) a.norm_idx[k] = prm->norm_idx[k];
-      }
       const int B = 256;
       hctu_con2pri<R,P,NC,LR><<< hctu_grid( NX3, n, B ), B, 0, st >>>( a );
       if ( cfg.char_reconstruction ) hctu_recon<R,P,RS,NC,1,LR><<< hctu_grid( NF3, n, B, 3 ), B, 0, st >>>( a );
@@ -612,8 +349,14 @@ size_t ctu_hydro_scratch_bytes_per_pg( int precision, int ncomp, int lr_scheme )
 
 // one hydro CTU solve of npg patch groups in chunks of scratch_bytes / ctu_hydro_scratch_bytes_per_pg
 int ctu_hydro_solve( const gb_fluid_config &cfg, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
-                     const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, cudaStream_t st )
+                     const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, int *status, cudaStream_t st )
 {
+   if ( ctu_hydro_fused( cfg, npg ) )
+   {
+      if ( cfg.precision == GB_PREC_FP64 )  return ctu_fused_fp64 ( cfg, flu_in, flu_out, flux, npg, prm, status, st );
+      if ( cfg.precision == GB_PREC_MIXED ) return ctu_fused_mixed( cfg, flu_in, flu_out, flux, npg, prm, status, st );
+      return ctu_fused_fp32( cfg, flu_in, flu_out, flux, npg, prm, status, st );
+   }
    if ( cfg.precision == GB_PREC_FP64 )
       return hctu_solve_lr<double,P_FP64>( cfg, flu_in, flu_out, flux, de, npg, prm, scratch, scratch_bytes, st );
    if ( cfg.precision == GB_PREC_MIXED )

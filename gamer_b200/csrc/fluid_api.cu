@@ -44,7 +44,8 @@ size_t ctu_ppm_mhd_scratch_bytes_per_pg( int precision );
 size_t mhm_ppm_mhd_scratch_bytes_per_pg( int precision );
 size_t ctu_hydro_scratch_bytes_per_pg( int precision, int ncomp, int lr_scheme );
 int ctu_hydro_solve( const gb_fluid_config &cfg, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
-                     const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, cudaStream_t st );
+                     const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, int *status, cudaStream_t st );
+bool ctu_hydro_fused( const gb_fluid_config &cfg, int npg );
 int ctu_solve( const gb_fluid_config &cfg, const void *flu_in, const void *mag_in, void *flu_out, void *mag_out,
                void *flux, void *ele, int npg, const gb_fluid_params *prm, void *scratch, size_t scratch_bytes,
                cudaStream_t st );
@@ -373,7 +374,8 @@ int solve_host_ctu( gb_fluid_solver *s, const void *flu_in, void *flu_out, const
               cudaMemcpyAsync( s->d_de[q], de_out + p0*bd, n*bd, cudaMemcpyHostToDevice, st ) != cudaSuccess )
             return GB_E_CUDA;
          rc = gb::ctu_hydro_solve( s->cfg, s->d_in[q], s->d_out[q], prm->store_flux ? s->d_flux[q] : nullptr,
-                                   ( dual && de_out ) ? s->d_de[q] : nullptr, n, prm, s->d_scratch[q], scratch_chunk, st );
+                                   ( dual && de_out ) ? s->d_de[q] : nullptr, n, prm, s->d_scratch[q], scratch_chunk,
+                                   s->d_status, st );
       }
       if ( rc != GB_OK ) return rc;
       if ( dual && de_out && !mhd &&
@@ -783,12 +785,12 @@ int gb_fluid_solve_device( gb_fluid_solver *s, const void *flu_in, void *flu_out
    }
    if ( is_ctu( s ) )
    {
-      const int chunk = ( npg < mhd_chunk( s ) ) ? npg : mhd_chunk( s );
-      rc = ensure_scratch( s, 0, chunk );
-      if ( rc != GB_OK ) return rc;
+      // the plane-streaming kernel needs no scratch
+      const int chunk = gb::ctu_hydro_fused( s->cfg, npg ) ? 0 : ( npg < mhd_chunk( s ) ) ? npg : mhd_chunk( s );
+      if ( chunk > 0 && ( rc = ensure_scratch( s, 0, chunk ) ) != GB_OK ) return rc;
       s->last = (cudaStream_t)stream;
       return gb::ctu_hydro_solve( s->cfg, flu_in, flu_out, prm->store_flux ? flux : nullptr, de_out, npg, prm,
-                                  s->d_scratch[0], ctu_per_pg( s )*(size_t)chunk, (cudaStream_t)stream );
+                                  s->d_scratch[0], ctu_per_pg( s )*(size_t)chunk, s->d_status, (cudaStream_t)stream );
    }
    if ( is_rp( s ) )
    {
