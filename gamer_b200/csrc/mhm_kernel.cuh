@@ -54,6 +54,9 @@ struct MhmArgs {
    R        dt[GB_MAX_LEVEL], dh[GB_MAX_LEVEL];
    int      nnorm;                           // NormPassive: number of listed passive scalars (0 = off)
    int      norm_idx[4];                     // NormIdx (passive indices, no repeats)
+   // work items: the patch groups below nwhole as a whole, the others in slabs of PS2 >> slab_log2
+   // output planes (mhm_plan)
+   int      nitem, nwhole, slab_log2;
 };
 
 // shared-memory carve-up (byte offsets), identical on host and device
@@ -287,21 +290,25 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
    }
    __syncthreads();
 
-   // ring slot, and mbarrier phase parity, of cc plane c during sweep number `pass` of this CTA
-   // (every sweep loads planes 0..N-1 in order, so slot q is used cnt(q) times per sweep)
-   uint32_t pass = 0;
+   // ring slot, and mbarrier phase parity, of cc plane c of a sweep of this CTA (a sweep loads its
+   // planes 0..NZ-1 in order, so slot q is used ( NZ - q + NSLOT - 1 )/NSLOT times)
+   uint32_t phase = 0;                    // bit q: parity of slot q's first use in this sweep
    auto slot_of   = [&]( int c ) { return c % NSLOT; };
-   auto parity_of = [&]( int c ) {
-      const int q = c % NSLOT;
-      const uint32_t cnt = ( N - q + NSLOT - 1 )/NSLOT;
-      return ( pass*cnt + (uint32_t)( c/NSLOT ) ) & 1u;
-   };
+   auto parity_of = [&]( int c ) { return ( ( phase >> ( c % NSLOT ) ) + (uint32_t)( c/NSLOT ) ) & 1u; };
    // primitive plane c, shifted to the scheme window: element (ci, cj) of variable v is
    // plane(c)[v*nin2 + cj*nin + ci]
    auto plane = [&]( int c ) { return s_pln + slot_of( c )*NC*nin2 + sh*nin + sh; };
 
-   for (int pg = blockIdx.x; pg < a.npg; pg += gridDim.x)
+   for (int item = blockIdx.x; item < a.nitem; item += gridDim.x)
    {
+      // the patch group and its output planes [o0, o0 + np): all cc and fc plane numbers below count
+      // from the first one this slab needs
+      const bool whole = ( item < a.nwhole );
+      const int part = item - a.nwhole;
+      const int pg = whole ? item : a.nwhole + ( part >> a.slab_log2 );
+      const int np = whole ? PS2 : PS2 >> a.slab_log2;
+      const int o0 = whole ? 0 : ( part & ( ( 1 << a.slab_log2 ) - 1 ) )*np;
+      const int NZ = np + 2*G;
       int lv = 0;
       while ( lv + 1 < a.nlevel && pg >= a.level_start[lv + 1] ) lv++;
       const R dt = a.dt[lv], dh = a.dh[lv];
@@ -318,7 +325,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
          fence_proxy_async();
          mbar_expect_tx( &bar[q], plane_bytes );
          for (int v=0; v<NC; v++)
-            bulk_g2s( s_pln + ( q*NC + v )*nin2, g_in + (size_t)v*nin*nin2 + (size_t)( c + sh )*nin2,
+            bulk_g2s( s_pln + ( q*NC + v )*nin2, g_in + (size_t)v*nin*nin2 + (size_t)( c + o0 + sh )*nin2,
                       nin2*sizeof(R), &bar[q] );
       };
 
@@ -367,7 +374,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
       // flight (planes c to c + AHEAD - 1), then this CTA gives up
       auto bail = [&]( int c ) {
          if ( tid == 0 )
-            for (int q = c; q < c + AHEAD && q < N; q++) mbar_wait_bounded( &bar[slot_of( q )], parity_of( q ) );
+            for (int q = c; q < c + AHEAD && q < NZ; q++) mbar_wait_bounded( &bar[slot_of( q )], parity_of( q ) );
          __syncthreads();
       };
       // phase-A conversion: the threads from conv0 on (those without an interior column when the
@@ -393,7 +400,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
          R zup[CARRY_SMEM ? 1 : NC];
          A fzp[CARRY_SMEM ? 1 : NC];
 
-         for (int t = 0; t < N; t++)
+         for (int t = 0; t < NZ; t++)
          {
             const int kf = t - NG - LAG;
             const int cz = kf + NG;                                  // centre cc plane
@@ -402,7 +409,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
             if ( kf >= 0 )
             {
                const R *pc = plane( cz ), *pm = plane( cz - 1 ), *pp = plane( cz + 1 );
-               const bool edge = ( kf == 0 || kf == NFC - 1 );
+               const bool edge = ( kf == 0 || kf == np + 1 );
                const int ncell = edge ? PS2*PS2 : PS2*PS2 + 4*PS2;
                for (int e = tid; e < ncell; e += nth)
                {
@@ -416,7 +423,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                      else               { i = 1 + r;   j = NFC - 1; }
                   }
                   const int ce = ( j + NG )*nin + ( i + NG );
-                  const size_t gidx = (size_t)( cz + sh )*nin2 + ( j + NG + sh )*nin + ( i + NG + sh );
+                  const size_t gidx = (size_t)( cz + o0 + sh )*nin2 + ( j + NG + sh )*nin + ( i + NG + sh );
                   R cc[NC], nl[NC], nr[NC];
                   R fcon[6][NC], fpres[6], acc[NC];
                   bool reset;
@@ -532,7 +539,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
 #                       pragma unroll
                         for (int v=0; v<NC; v++) zl[v] = CARRY_SMEM ? s_czu[v*PS2*PS2 + col] : zup[CARRY_SMEM ? 0 : v];
                         riemann<RS,2,P,NC>( ph, zl, fcon[4], F );
-                        const int ko = kf - 1;
+                        const int ko = o0 + kf - 1;      // a face between two slabs is stored by both, alike
                         if ( g_flux != nullptr && ( ko & 7 ) == 0 )
                         {
                            R *dst = g_flux + (size_t)( ( 6 + ( ko >> 3 ) )*NC )*PS2*PS2 + col;
@@ -542,7 +549,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                         if ( kf >= 2 )
                         {
                            // output plane o = kf-2: its x/y fluxes are those of fc plane kf-1
-                           const int o = kf - 2, oi0 = i - 1, oj0 = j - 1;
+                           const int o = o0 + kf - 2, oi0 = i - 1, oj0 = j - 1;
                            const FP *fx = s_flx, *fy = s_fly;
                            // U_in of the output cell: the input at offset FLU_GHOST_SIZE (MHM_RP: the
                            // conserved 22^3 input, FLU_GHOST_SIZE = 3)
@@ -599,18 +606,18 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                }
             }
             if constexpr ( CONV_A )
-               if ( t + 1 < N && tid >= conv0 ) convert( t + 1, tid - conv0, nth - conv0 );
+               if ( t + 1 < NZ && tid >= conv0 ) convert( t + 1, tid - conv0, nth - conv0 );
             __syncthreads();
             // the slot of the oldest live plane is free now: prefetch cc plane t+AHEAD into it
-            if ( tid == 0 && t + AHEAD < N ) issue( t + AHEAD );
+            if ( tid == 0 && t + AHEAD < NZ ) issue( t + AHEAD );
 
             // (B) x (17x16) and y (16x17) Riemann problems of plane kf for kf in [1,17); conversion
             // of cc plane t+1
             int nrm = 0;
-            if ( kf >= 1 && kf <= NFC - 2 )
+            if ( kf >= 1 && kf <= np )
             {
                const int nx = PS2*NFLX;
-               const int ko = kf - 1;          // k index of the x/y fluxes
+               const int ko = o0 + kf - 1;     // k index of the x/y fluxes
                FP *flx = s_flx, *fly = s_fly;
                if constexpr ( X2 )
                {
@@ -711,12 +718,12 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
             }
             // the cells are dealt out starting at the first thread with one Riemann problem fewer
             if constexpr ( !CONV_A )
-               if ( t + 1 < N ) convert( t + 1, ( tid + nth - nrm % nth ) % nth, nth );
+               if ( t + 1 < NZ ) convert( t + 1, ( tid + nth - nrm % nth ) % nth, nth );
             __syncthreads();
             if ( s_flag[1] ) { bail( t + 1 );  return; }
          } // for t
 
-         pass++;
+         for (int q=0; q<NSLOT; q++) phase ^= ( ( ( NZ - q + NSLOT - 1 )/NSLOT ) & 1u ) << q;
          const bool fail = ( s_flag[0] != 0 );
          iter++;
          again = fail && iter <= a.minmod_maxiter;
@@ -731,7 +738,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
          else if ( !fail && tid == 0 && a.pg_fail != nullptr ) a.pg_fail[pg] = 0;
          __syncthreads();
       } while ( again );
-   } // for pg
+   } // for item
 }
 
 } // namespace gb
