@@ -78,6 +78,7 @@ struct CtuArgs {
    int npg;
    int limiter;
    int ec_pg;        // EMF elements per patch group (3 components at the largest stride)
+   int fcf_pg;       // flux elements per patch group (the region that holds the fluxes)
    R coeff, dt, dh;
    Phys<R> ph;
 };
@@ -137,11 +138,12 @@ __global__ void ctu_con2pri( const __grid_constant__ CtuArgs<R> a )
 // eigenvectors along D), or PPM from the limited slopes of the cell and its two neighbours (each
 // limited, with CH, in its own cell's wave amplitudes); CPU_Shared_DataReconstruction.cpp:386-430,
 // :870-907, :1080-1130
-template <int D, int CH, int LR, typename R>
+// GMM: generalized MinMod with theta < 2 built in (its PLM clamps never act); otherwise the run-time limiter
+template <int D, int CH, int LR, bool GMM, typename R>
 GB_DEV void mhd_face_values( const CtuArgs<R> &a, const R *pri, int PL, int c, int st, const R *cc,
                              const R (&LE)[7][7], const R (&RE)[7][7], R (&fl)[NM], R (&fr)[NM] )
 {
-   const int NX3 = PL;
+   const int NX3 = PL, lim = GMM ? LIM_GMINMOD : a.limiter;
    const int dcc[3] = { st, st, st };
    if constexpr ( LR == LR_PPM )
    {
@@ -158,13 +160,13 @@ GB_DEV void mhd_face_values( const CtuArgs<R> &a, const R *pri, int PL, int c, i
          {
             R e_[7], L_[7][7], R_[7][7];
             mhd_eigen<D>( a.ph, pm1, e_, L_, R_ );
-            mhd_char_limited_slopes<D>( a.ph, L_, R_, pm2, pm1, cc, a.limiter, a.coeff, sl );
+            mhd_char_limited_slopes<D>( a.ph, L_, R_, pm2, pm1, cc, lim, a.coeff, sl );
          }
-         mhd_char_limited_slopes<D>( a.ph, LE, RE, pm1, cc, pp1, a.limiter, a.coeff, sc );
+         mhd_char_limited_slopes<D>( a.ph, LE, RE, pm1, cc, pp1, lim, a.coeff, sc );
          {
             R e_[7], L_[7][7], R_[7][7];
             mhd_eigen<D>( a.ph, pp1, e_, L_, R_ );
-            mhd_char_limited_slopes<D>( a.ph, L_, R_, cc, pp1, pp2, a.limiter, a.coeff, sr );
+            mhd_char_limited_slopes<D>( a.ph, L_, R_, cc, pp1, pp2, lim, a.coeff, sr );
          }
       }
       else
@@ -173,21 +175,21 @@ GB_DEV void mhd_face_values( const CtuArgs<R> &a, const R *pri, int PL, int c, i
          for (int v=0; v<NM; v++)
          {
             const R *q = pri + v*NX3 + c;
-            sl[v] = limit_slope( q[-2*dcc[D]], q[-dcc[D]], q[0],        a.limiter, a.coeff );
-            sc[v] = limit_slope( q[-dcc[D]],   q[0],       q[dcc[D]],   a.limiter, a.coeff );
-            sr[v] = limit_slope( q[0],         q[dcc[D]],  q[2*dcc[D]], a.limiter, a.coeff );
+            sl[v] = limit_slope( q[-2*dcc[D]], q[-dcc[D]], q[0],        lim, a.coeff );
+            sc[v] = limit_slope( q[-dcc[D]],   q[0],       q[dcc[D]],   lim, a.coeff );
+            sr[v] = limit_slope( q[0],         q[dcc[D]],  q[2*dcc[D]], lim, a.coeff );
          }
       }
 #     pragma unroll
       for (int v=0; v<NM; v++)
-         ppm_faces( pri[v*NX3 + c - dcc[D]], cc[v], pri[v*NX3 + c + dcc[D]], sl[v], sc[v], sr[v], a.limiter, fl[v], fr[v] );
+         ppm_faces( pri[v*NX3 + c - dcc[D]], cc[v], pri[v*NX3 + c + dcc[D]], sl[v], sc[v], sr[v], lim, fl[v], fr[v] );
    }
    else if constexpr ( CH )
    {
       R cl[NM], cr[NM], s[NM];
 #     pragma unroll
       for (int v=0; v<NM; v++) { cl[v] = pri[v*NX3 + c - dcc[D]];  cr[v] = pri[v*NX3 + c + dcc[D]]; }
-      mhd_char_limited_slopes<D>( a.ph, LE, RE, cl, cc, cr, a.limiter, a.coeff, s );
+      mhd_char_limited_slopes<D>( a.ph, LE, RE, cl, cc, cr, lim, a.coeff, s );
 #     pragma unroll
       for (int v=0; v<NM; v++) plm_clamped_faces( cl[v], cc[v], cr[v], s[v], fl[v], fr[v] );
    }
@@ -197,7 +199,7 @@ GB_DEV void mhd_face_values( const CtuArgs<R> &a, const R *pri, int PL, int c, i
       for (int v=0; v<NM; v++)
       {
          const R l = pri[v*NX3 + c - dcc[D]], r = pri[v*NX3 + c + dcc[D]];
-         plm_faces( l, cc[v], r, a.limiter, a.coeff, true, fl[v], fr[v] );
+         plm_faces( l, cc[v], r, lim, a.coeff, !GMM, fl[v], fr[v] );
       }
    }
 }
@@ -206,7 +208,7 @@ GB_DEV void mhd_face_values( const CtuArgs<R> &a, const R *pri, int PL, int c, i
 // (each, with CH, limited in its own cell's MHD wave amplitudes), and the tracing of the parabola:
 // each wave's correction carries the curvature term dfc6 = 6 (cc - (fL + fR)/2)
 // (CPU_Shared_DataReconstruction.cpp:870-907, :1080-1290)
-template <int D, int CH, int LR, typename R>
+template <int D, int CH, int LR, bool GMM, typename R>
 GB_DEV void ctu_recon_dir( const CtuArgs<R> &a, const R *pri, const R *bin, const R *cc,
                            int ci, int cj, int ck, R (&fcon)[2][NM] )
 {
@@ -216,51 +218,45 @@ GB_DEV void ctu_recon_dir( const CtuArgs<R> &a, const R *pri, const R *bin, cons
    constexpr int t1 = ( D + 1 ) % 3, t2 = ( D + 2 ) % 3;
    const int dcc[3] = { 1, N, N*N };
    const int c = idx3( ci, cj, ck, N, N );
-   R ev[7], LE[7][7], RE[7][7];
-   mhd_eigen<D>( a.ph, cc, ev, LE, RE );
    R fl[NM], fr[NM];
-   mhd_face_values<D,CH,LR>( a, pri, NX3, c, dcc[D], cc, LE, RE, fl, fr );
-   // characteristic tracing with all waves (HLL solvers: HLL_NO_REF_STATE, HLL_INCLUDE_ALL_WAVES)
+   {
+      // (the eigenvectors serve the characteristic limiting alone)
+      R ev[7], LE[7][7], RE[7][7];
+      if constexpr ( CH ) mhd_eigen<D>( a.ph, cc, ev, LE, RE );
+      mhd_face_values<D,CH,LR,GMM>( a, pri, NX3, c, dcc[D], cc, LE, RE, fl, fr );
+   }
+   // characteristic tracing with all waves (HLL solvers: HLL_NO_REF_STATE, HLL_INCLUDE_ALL_WAVES): the
+   // sum over the seven waves of a polynomial of the eigenvalue, linear (PLM) or quadratic (PPM), is
+   // that polynomial of the primitive-variable Jacobian (mhd_jacobian)
    const R dt_dh2 = R(0.5)*a.dt/a.dh;
    const int wv[7] = { 0, M::n, M::t1, M::t2, 4, M::b1, M::b2 };   // wave index -> storage index
    R dfc[7], corr[7], corl[7];
 #  pragma unroll
-   for (int q=0; q<7; q++) { dfc[q] = fr[wv[q]] - fl[wv[q]];  corr[q] = R(0);  corl[q] = R(0); }
+   for (int q=0; q<7; q++) dfc[q] = fr[wv[q]] - fl[wv[q]];
    if constexpr ( LR == LR_PPM )
    {
-      R dfc6[7];
+      // each wave's correction carries the curvature term dfc6 = 6 (cc - (fL + fR)/2)
+      R d6[7], e[7], y6[7], yy6[7];
 #     pragma unroll
-      for (int q=0; q<7; q++) dfc6[q] = R(6)*( cc[wv[q]] - R(0.5)*( fl[wv[q]] + fr[wv[q]] ) );
+      for (int q=0; q<7; q++) d6[q] = R(6)*( cc[wv[q]] - R(0.5)*( fl[wv[q]] + fr[wv[q]] ) );
+      mhd_jacobian<D>( a.ph, cc, d6, y6 );
+      mhd_jacobian<D>( a.ph, cc, y6, yy6 );
+      mhd_jacobian<D>( a.ph, cc, dfc, e );
+      const R c2 = R(4.0/3.0)*dt_dh2*dt_dh2;
 #     pragma unroll
-      for (int m=0; m<7; m++)
+      for (int q=0; q<7; q++)
       {
-         const R cC = -dt_dh2*ev[m], cD = R(-4.0/3.0)*( cC*cC );
-         R cfl = R(0), cfr = R(0);
-#        pragma unroll
-         for (int q=0; q<7; q++)
-         {
-            cfl += LE[m][q]*( cC*( dfc[q] + dfc6[q] ) + cD*dfc6[q] );
-            cfr += LE[m][q]*( cC*( dfc[q] - dfc6[q] ) + cD*dfc6[q] );
-         }
-#        pragma unroll
-         for (int q=0; q<7; q++) { corl[q] = corl[q] + mul_rn( cfl, RE[m][q] );  corr[q] = corr[q] + mul_rn( cfr, RE[m][q] ); }
+         const R cur = -c2*yy6[q];
+         corl[q] = cur - dt_dh2*( e[q] + y6[q] );
+         corr[q] = cur - dt_dh2*( e[q] - y6[q] );
       }
    }
    else
    {
+      R y[7];
+      mhd_jacobian<D>( a.ph, cc, dfc, y );
 #     pragma unroll
-      for (int m=0; m<7; m++)
-      {
-         R cf = R(0);
-#        pragma unroll
-         for (int q=0; q<7; q++) cf += LE[m][q]*dfc[q];
-         cf *= -dt_dh2*ev[m];
-         // uncontracted: the Alfven pair (modes 1 and 5) cancels exactly in B_t when B = 0
-#        pragma unroll
-         for (int q=0; q<7; q++) corr[q] = corr[q] + mul_rn( cf, RE[m][q] );
-      }
-#     pragma unroll
-      for (int q=0; q<7; q++) corl[q] = corr[q];
+      for (int q=0; q<7; q++) corl[q] = corr[q] = -dt_dh2*y[q];
    }
    // MHD source terms of the transverse B (CPU_Shared_DataReconstruction.cpp:593-620)
    const int ib[3] = { idx_b( 0, ci, cj, ck, N ), idx_b( 1, ci, cj, ck, N ), idx_b( 2, ci, cj, ck, N ) };
@@ -300,9 +296,9 @@ __global__ void __launch_bounds__( 256, ( sizeof(R) == 8 ) ? 1 : ( ( CH || LR ==
       R cc[NM], fcon[2][NM];
 #     pragma unroll
       for (int v=0; v<NM; v++) cc[v] = pri[v*plane_of( N ) + c];
-      if      ( d == 0 ) ctu_recon_dir<0,CH,LR>( a, pri, bin, cc, ci, cj, ck, fcon );
-      else if ( d == 1 ) ctu_recon_dir<1,CH,LR>( a, pri, bin, cc, ci, cj, ck, fcon );
-      else               ctu_recon_dir<2,CH,LR>( a, pri, bin, cc, ci, cj, ck, fcon );
+      if      ( d == 0 ) ctu_recon_dir<0,CH,LR,false>( a, pri, bin, cc, ci, cj, ck, fcon );
+      else if ( d == 1 ) ctu_recon_dir<1,CH,LR,false>( a, pri, bin, cc, ci, cj, ck, fcon );
+      else               ctu_recon_dir<2,CH,LR,false>( a, pri, bin, cc, ci, cj, ck, fcon );
       R *fcv = a.fcv + (size_t)pg*6*NM*NF3;
 #     pragma unroll
       for (int q=0; q<2; q++)
@@ -313,6 +309,25 @@ __global__ void __launch_bounds__( 256, ( sizeof(R) == 8 ) ? 1 : ( ( CH || LR ==
 
 // ---- K2/K7: Riemann fluxes (Hydro_ComputeFlux, CPU_Shared_ComputeFlux.cpp:113-376) ----------
 // half step: NSkip_N = NSkip_T = 0, stride 20; full step: NSkip_N = NSkip_T = 1, stride 18
+// coarse-fine flux planes (Hydro_StoreIntFlux with MHD, CPU_Shared_ComputeFlux.cpp:391-450)
+template <int D, typename R>
+GB_DEV void ctu_store_planes( const CtuArgs<R> &a, int pg, int fi, int fj, int fk, const R (&F)[NM] )
+{
+   if ( a.flux == nullptr ) return;
+   const int fl[3] = { fi, fj, fk };
+   const int nrm = fl[D];
+   const int t1 = fl[( D + 1 ) % 3], t2 = fl[( D + 2 ) % 3];
+   if ( ( nrm & 7 ) == 0 && t1 >= 1 && t1 <= PS2 && t2 >= 1 && t2 <= PS2 )
+   {
+      // idx_out: transverse index with the smaller axis number is the fastest
+      const int a0 = ( D == 0 ) ? fj : fi, a1 = ( D == 2 ) ? fj : fk;
+      const int io = ( a1 - 1 )*PS2 + ( a0 - 1 );
+      R *dst = a.flux + (size_t)pg*9*5*PS2*PS2 + (size_t)( 3*D + nrm/PS1 )*5*PS2*PS2 + io;
+#     pragma unroll
+      for (int v=0; v<5; v++) dst[v*PS2*PS2] = F[v];
+   }
+}
+
 template <int D, typename R, int P>
 GB_DEV void ctu_face( const CtuArgs<R> &a, int pg, int fi, int fj, int fk, int skip, int nflux, bool store_int )
 {
@@ -328,22 +343,7 @@ GB_DEV void ctu_face( const CtuArgs<R> &a, int pg, int fi, int fj, int fk, int s
    const int ix = idx3( fi, fj, fk, nflux, nflux );
 #  pragma unroll
    for (int v=0; v<NM; v++) fcf[( D*NM + v )*NF3 + ix] = F[v];
-   // coarse-fine flux planes (Hydro_StoreIntFlux with MHD, CPU_Shared_ComputeFlux.cpp:391-450)
-   if ( store_int && a.flux != nullptr )
-   {
-      const int fl[3] = { fi, fj, fk };
-      const int nrm = fl[D];
-      const int t1 = fl[( D + 1 ) % 3], t2 = fl[( D + 2 ) % 3];
-      if ( ( nrm & 7 ) == 0 && t1 >= 1 && t1 <= PS2 && t2 >= 1 && t2 <= PS2 )
-      {
-         // idx_out: transverse index with the smaller axis number is the fastest
-         const int a0 = ( D == 0 ) ? fj : fi, a1 = ( D == 2 ) ? fj : fk;
-         const int io = ( a1 - 1 )*PS2 + ( a0 - 1 );
-         R *dst = a.flux + (size_t)pg*9*5*PS2*PS2 + (size_t)( 3*D + nrm/PS1 )*5*PS2*PS2 + io;
-#        pragma unroll
-         for (int v=0; v<5; v++) dst[v*PS2*PS2] = F[v];
-      }
-   }
+   if ( store_int ) ctu_store_planes<D>( a, pg, fi, fj, fk, F );
 }
 
 // FP32: 3 CTAs of 256 threads per SM (80 registers, no spills): MHD step 2.08 -> 1.94 ms per
@@ -405,7 +405,7 @@ GB_DEV void ctu_emf_dir( const CtuArgs<R> &a, int pg, int q )
       const int ifl = idx3( ie + sf[0], je + sf[1], ke + sf[2], nflux, nflux );
       const int ip  = idx3( ie + sf[0] + off_pri, je + sf[1] + off_pri, ke + sf[2] + off_pri, npri, npri );
       const int dfl[3] = { 1, nflux, nflux*nflux }, dpr[3] = { 1, npri, npri*npri };
-      const R *F = ( G == 2 ) ? a.fcv + (size_t)pg*6*NM*NF3 : a.fcf + (size_t)pg*3*NM*NF3;
+      const R *F = ( G == 2 ) ? a.fcv + (size_t)pg*6*NM*NF3 : a.fcf + (size_t)pg*a.fcf_pg;
       const R *W = a.pri + (size_t)pg*NM*pri_plane;
       auto f = [&]( int dir, int v, int idx ) { return F[( dir*NM + v )*fplane + idx]; };
       auto w = [&]( int v, int idx ) { return W[v*pri_plane + idx]; };
@@ -499,20 +499,17 @@ __global__ void ctu_bupdate( const __grid_constant__ CtuArgs<R> a, R *bout_base,
 }
 
 // ---- K5: transverse-gradient correction (Hydro_TGradientCorrection, CPU_FluidSolver_CTU.cpp:368-599) ----
+// the two face states q0, q1 along D of face-state cell (i0 + 1, j0 + 1, k0 + 1), in place
 template <int D, typename R, int P, int NXI = ctu::NX>
-GB_DEV void ctu_tgrad_dir( const CtuArgs<R> &a, int pg, int i0, int j0, int k0 )
+GB_DEV void ctu_correct( const CtuArgs<R> &a, int pg, int i0, int j0, int k0, R (&q0)[NM], R (&q1)[NM] )
 {
    using namespace ctu;
    typedef MDir<D> M;
    constexpr int T1 = ( D + 1 ) % 3, T2 = ( D + 2 ) % 3;
    const int dfl[3] = { 1, NF, NF*NF };
    const int f = idx3( i0 + 1, j0 + 1, k0 + 1, NF, NF );
-   R *fcv = a.fcv + (size_t)pg*6*NM*NF3;
    const R *F = a.fcf + (size_t)pg*3*NM*NF3;
    const R dt_dh2 = R(0.5)*a.dt/a.dh;
-   R q0[NM], q1[NM];
-#  pragma unroll
-   for (int v=0; v<NM; v++) { q0[v] = fcv[( 2*D*NM + v )*NF3 + f];  q1[v] = fcv[( ( 2*D + 1 )*NM + v )*NF3 + f]; }
 #  pragma unroll
    for (int v=0; v<5; v++)
    {
@@ -574,6 +571,18 @@ GB_DEV void ctu_tgrad_dir( const CtuArgs<R> &a, int pg, int i0, int j0, int k0 )
       e = eint_con_mhd<P>( q1[0], R(1)/q1[0], q1[1], q1[2], q1[3], q1[4], em1 );
       if ( e == e && e < a.ph.min_eint ) q1[4] = q1[4] - e + a.ph.min_eint;
    }
+}
+
+template <int D, typename R, int P, int NXI = ctu::NX>
+GB_DEV void ctu_tgrad_dir( const CtuArgs<R> &a, int pg, int i0, int j0, int k0 )
+{
+   using namespace ctu;
+   const int f = idx3( i0 + 1, j0 + 1, k0 + 1, NF, NF );
+   R *fcv = a.fcv + (size_t)pg*6*NM*NF3;
+   R q0[NM], q1[NM];
+#  pragma unroll
+   for (int v=0; v<NM; v++) { q0[v] = fcv[( 2*D*NM + v )*NF3 + f];  q1[v] = fcv[( ( 2*D + 1 )*NM + v )*NF3 + f]; }
+   ctu_correct<D,R,P,NXI>( a, pg, i0, j0, k0, q0, q1 );
 #  pragma unroll
    for (int v=0; v<NM; v++) { fcv[( 2*D*NM + v )*NF3 + f] = q0[v];  fcv[( ( 2*D + 1 )*NM + v )*NF3 + f] = q1[v]; }
 }
@@ -591,6 +600,74 @@ __global__ void __launch_bounds__( 256, ( sizeof(R) == 8 ) ? 1 : 4 ) ctu_tgrad( 
       GB_CTU_DIR( GB_TG )
 #     undef GB_TG
    }
+}
+
+// ---- face states and Riemann fluxes of one slice in one kernel (CTU, limiting in primitive variables) ----
+// FULL 0: the half-step fluxes (reconstruction with tracing of 20 x 20 cells, 19 x 20 faces); FULL 1: the
+// full-step fluxes (the same reconstruction of the inner 18 x 18 cells, their transverse-gradient
+// correction, 17 x 18 faces, with the coarse-fine planes).  One CTA takes one slice of cells that
+// contains the direction D of the faces: an x-y plane for D = x and y, an x-z plane for D = z.  The
+// face states go through shared memory, 16 values a cell; they are formed twice (the tracing takes two
+// sparse products with the Jacobian) instead of being stored, corrected in place and read again:
+// of ~12 MB of global traffic per patch group (FP32) that leaves ~6 MB.  2 CTAs of 416 threads per SM
+// (72 registers).  The whole step, with the tracing by the Jacobian, FP32: PLM, 2048 patch groups
+// 6587 -> 4818 us; PPM, 300: 1880 -> 1063; mixed PLM, 300: 1083 -> 853; 64: 284 -> 208.  In FP64 (one CTA per
+// SM) the slices were slower than the stored face states, and the characteristic limiting needs both
+// bases twice: those two keep the kernels above.
+constexpr int SL_THREADS = 416;
+
+template <int D, typename R, int P, int LR, int FULL, bool GMM>
+GB_DEV void ctu_slice( const CtuArgs<R> &a, int pg, int slice, R *s_fc )
+{
+   using namespace ctu;
+   constexpr int NXI = ( LR == LR_PPM ) ? NX + 2 : NX, LRGc = flg_of( NXI ) - 2;
+   constexpr int NC_ = FULL ? NF - 2 : NF, NFc = NC_*NC_, o = FULL ? 1 : 0;      // cells of the slice, first cell
+   // element (u, w) of the slice: u along x, w along y (D = x, y) or z (D = z); the faces of D = x
+   // run along u, the others along w
+   for (int t = threadIdx.x; t < NFc; t += SL_THREADS)
+   {
+      const int u = t % NC_, w = t / NC_;
+      const int fi = u + o, fj = ( D == 2 ? slice : w ) + o, fk = ( D == 2 ? w : slice ) + o;   // face-state cell
+      const R *pri = a.pri + (size_t)pg*NM*plane_of( NXI );
+      const R *bin = a.bin + (size_t)pg*3*nbin_of( NXI );
+      const int ci = fi + LRGc, cj = fj + LRGc, ck = fk + LRGc, c = idx3( ci, cj, ck, NXI, NXI );
+      R cc[NM], q[2][NM];
+#     pragma unroll
+      for (int v=0; v<NM; v++) cc[v] = pri[v*plane_of( NXI ) + c];
+      ctu_recon_dir<D,0,LR,GMM>( a, pri, bin, cc, ci, cj, ck, q );
+      if constexpr ( FULL ) ctu_correct<D,R,P,NXI>( a, pg, fi - 1, fj - 1, fk - 1, q[0], q[1] );
+#     pragma unroll
+      for (int v=0; v<NM; v++) { s_fc[v*NFc + t] = q[0][v];  s_fc[( NM + v )*NFc + t] = q[1][v]; }
+   }
+   __syncthreads();
+   for (int t = threadIdx.x; t < ( NC_ - 1 )*NC_; t += SL_THREADS)
+   {
+      constexpr int e0 = ( D == 0 ) ? NC_ - 1 : NC_, step = ( D == 0 ) ? 1 : NC_;
+      const int u = t % e0, w = t / e0, f = w*NC_ + u;
+      R L[NM], Rr[NM], F[NM];
+#     pragma unroll
+      for (int v=0; v<NM; v++) { L[v] = s_fc[( NM + v )*NFc + f];  Rr[v] = s_fc[v*NFc + f + step]; }
+      riemann_mhd<D,P>( a.ph, L, Rr, F );
+      const int fi = u, fj = ( D == 2 ) ? slice : w, fk = ( D == 2 ) ? w : slice;
+      // the half-step fluxes stay in the flux region for the correction, the full-step ones go to the
+      // face-state region
+      R *fcf = FULL ? a.fcv + (size_t)pg*6*NM*NF3 : a.fcf + (size_t)pg*3*NM*NF3;
+      const int ix = idx3( fi, fj, fk, NC_, NC_ );
+#     pragma unroll
+      for (int v=0; v<NM; v++) fcf[( D*NM + v )*NF3 + ix] = F[v];
+      if constexpr ( FULL ) ctu_store_planes<D>( a, pg, fi, fj, fk, F );
+   }
+}
+
+template <typename R, int P, int LR, int FULL, bool GMM>
+__global__ void __launch_bounds__( SL_THREADS, 2 ) ctu_slice_flux( const __grid_constant__ CtuArgs<R> a )
+{
+   extern __shared__ __align__(16) unsigned char sl_smem[];
+   const int pg = blockIdx.z;
+   if ( a.active != nullptr && a.active[pg] == 0 ) return;
+#  define GB_SLICE( D ) ctu_slice<D,R,P,LR,FULL,GMM>( a, pg, blockIdx.x, (R*)sl_smem )
+   GB_CTU_DIR( GB_SLICE )
+#  undef GB_SLICE
 }
 
 // ---- K6: half-step cell-centred primitives (MHD_HalfStepPrimitive, CPU_Shared_ConstrainedTransport.cpp:629-700) ----
@@ -667,7 +744,7 @@ __global__ void ctu_update( const __grid_constant__ CtuArgs<R> a )
       const int ifl = idx3( io + 1, jo + 1, ko + 1, NFF, NFF );
       const int dfl[3] = { 1, NFF, NFF*NFF };
       const int iin = idx3( io + FLU, jo + FLU, ko + FLU, NXU, NXU );
-      const R *F = a.fcf + (size_t)pg*3*NM*NF3;
+      const R *F = a.fcf + (size_t)pg*a.fcf_pg;
       const R *u = a.in + (size_t)pg*5*NXU3;
       R *out = a.out + (size_t)pg*5*N3;
       R o[5];
@@ -818,7 +895,7 @@ GB_DEV void rp_recon_dir( const CtuArgs<R> &a, const R *hp, const R *bh, int hi,
    R fl[NM], fr[NM];
    R ev[7], LE[7][7], RE[7][7];
    if constexpr ( CH ) mhd_eigen<D>( a.ph, cc, ev, LE, RE );
-   mhd_face_values<D,CH,LR>( a, hp, HV3, c, dh3[D], cc, LE, RE, fl, fr );
+   mhd_face_values<D,CH,LR,false>( a, hp, HV3, c, dh3[D], cc, LE, RE, fl, fr );
    const int ib = idx_b( D, hi, hj, hk, HV );
    fl[M::bn] = bh[D*NBH_ + ib];
    fr[M::bn] = bh[D*NBH_ + ib + db_next( D, HV )];
@@ -934,7 +1011,7 @@ GB_DEV void mm_faces_dir( const CtuArgs<R> &a, const R *pri, const R *bin, const
    const int c = idx3( ic, jc, kc, N, N );
    R ev[7], LE[7][7], RE[7][7];
    if constexpr ( CH ) mhd_eigen<D>( a.ph, cc, ev, LE, RE );
-   mhd_face_values<D,CH,LR>( a, pri, PL, c, dcc[D], cc, LE, RE, wl, wr );
+   mhd_face_values<D,CH,LR,false>( a, pri, PL, c, dcc[D], cc, LE, RE, wl, wr );
    const int ib = idx_b( D, ic, jc, kc, N );
    wl[M::bn] = bin[D*NB + ib];
    wr[M::bn] = bin[D*NB + ib + db_next( D, N )];
@@ -1110,7 +1187,8 @@ size_t ctu_scratch_per_pg( size_t rsz, int scheme = GB_SCHEME_CTU, int nxi = ctu
 }
 
 // the CTU half step (reconstruction with tracing, half-step fluxes, EMFs and B, transverse-gradient
-// correction, half-step primitives) for PLM (FLU_NXT 22) or PPM (24)
+// correction, half-step primitives) for PLM (FLU_NXT 22) or PPM (24), with the face states
+// stored: FP64, and characteristic limiting, whose wave projections make them too dear to form twice
 template <typename R, int P, int LR>
 void ctu_half_step( const CtuArgs<R> &a, int charr, int n, cudaStream_t st )
 {
@@ -1118,12 +1196,30 @@ void ctu_half_step( const CtuArgs<R> &a, int charr, int n, cudaStream_t st )
    constexpr int NXI = ( LR == LR_PPM ) ? NX + 2 : NX;
    const int B = 256;
    if ( charr ) ctu_recon<R,P,1,LR><<< ctu_grid( NF3, n, B, 3 ), B, 0, st >>>( a );
-   else         ctu_recon<R,P,0,LR><<< ctu_grid( NF3, n, B, 3 ), B, 0, st >>>( a );
+   else if constexpr ( sizeof(R) == 8 ) ctu_recon<R,P,0,LR><<< ctu_grid( NF3, n, B, 3 ), B, 0, st >>>( a );
    ctu_flux<R,P,0><<< ctu_grid( ( NF - 1 )*NF*NF, n, B, 3 ), B, 0, st >>>( a );
    ctu_emf<R,0,NXI><<< ctu_grid( ( NHE - 1 )*NHE*NHE, n, B, 3 ), B, 0, st >>>( a );
    ctu_bupdate<R,0,NXI><<< ctu_grid( NBH, n, B, 3 ), B, 0, st >>>( a, a.bh, 3*(size_t)NBH, NBH, R(0.5)*a.dt );
    ctu_tgrad<R,P,NXI><<< ctu_grid( NHV*NHV*NHV, n, B, 3 ), B, 0, st >>>( a );
    ctu_halfprim<R,NXI><<< ctu_grid( NHV*NHV*NHV, n, B ), B, 0, st >>>( a );
+}
+
+// a CTU step up to the full-step fluxes with ctu_slice_flux (float, limiting in primitive variables)
+template <typename R, int P, int LR, bool GMM>
+cudaError_t ctu_slice_step( const CtuArgs<R> &a, int n, cudaStream_t st )
+{
+   using namespace ctu;
+   constexpr int NXI = ( LR == LR_PPM ) ? NX + 2 : NX;
+   constexpr int sm0 = 2*NM*NF*NF*(int)sizeof(R), sm1 = 2*NM*( NF - 2 )*( NF - 2 )*(int)sizeof(R);
+   const int B = 256;
+   cudaError_t e = cudaFuncSetAttribute( ctu_slice_flux<R,P,LR,0,GMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm0 );
+   if ( e != cudaSuccess ) return e;
+   ctu_slice_flux<R,P,LR,0,GMM><<< dim3( NF, 3, n ), SL_THREADS, sm0, st >>>( a );
+   ctu_emf<R,0,NXI><<< ctu_grid( ( NHE - 1 )*NHE*NHE, n, B, 3 ), B, 0, st >>>( a );
+   ctu_bupdate<R,0,NXI><<< ctu_grid( NBH, n, B, 3 ), B, 0, st >>>( a, a.bh, 3*(size_t)NBH, NBH, R(0.5)*a.dt );
+   ctu_slice_flux<R,P,LR,1,GMM><<< dim3( NF - 2, 3, n ), SL_THREADS, sm1, st >>>( a );
+   ctu_halfprim<R,NXI><<< ctu_grid( NHV*NHV*NHV, n, B ), B, 0, st >>>( a );
+   return cudaSuccess;
 }
 
 // the MHM_RP half step: first-order half-step fluxes of the input cells, their EMFs and the CT
@@ -1144,13 +1240,14 @@ void rp_half_step( const CtuArgs<R> &a, int charr, int n, cudaStream_t st )
 }
 
 // the full step shared by every scheme (the same faces, edges and half-step cells), on an input of
-// FLU_NXT NXI (20: MHM; 22: CTU+PLM, MHM_RP; 24: CTU+PPM)
+// FLU_NXT NXI (20: MHM; 22: CTU+PLM, MHM_RP; 24: CTU+PPM); flux: from the stored face states (otherwise the
+// fluxes are there already)
 template <typename R, int P, int NXI>
-void ctu_full_step( const CtuArgs<R> &af, int n, cudaStream_t st )
+void ctu_full_step( const CtuArgs<R> &af, int n, bool flux, cudaStream_t st )
 {
    using namespace ctu;
    const int B = 256;
-   ctu_flux<R,P,1><<< ctu_grid( ( NF - 3 )*( NF - 2 )*( NF - 2 ), n, B, 3 ), B, 0, st >>>( af );
+   if ( flux ) ctu_flux<R,P,1><<< ctu_grid( ( NF - 3 )*( NF - 2 )*( NF - 2 ), n, B, 3 ), B, 0, st >>>( af );
    ctu_emf<R,1,NXI><<< ctu_grid( ( NFE - 1 )*NFE*NFE, n, B, 3 ), B, 0, st >>>( af );
    if constexpr ( NXI == MNX )
       ctu_bupdate<R,3><<< ctu_grid( NBOUT, n, B, 3 ), B, 0, st >>>( af, af.bout, 3*(size_t)NBOUT, NBOUT, af.dt );
@@ -1194,6 +1291,7 @@ int ctu_solve_t( const gb_fluid_config &cfg, const void *in, const void *bin, vo
       a.ec   = take( (size_t)n*3*( rp ? rnec : (size_t)NEC ) );
       a.npg  = n;
       a.ec_pg = 3*( rp ? rnec : (size_t)NEC );
+      a.fcf_pg = 3*NM*NF3;
       a.limiter = prm->lr_limiter;
       a.coeff = (R)prm->minmod_coeff;
       a.dt = (R)prm->dt;  a.dh = (R)prm->dh;
@@ -1206,7 +1304,8 @@ int ctu_solve_t( const gb_fluid_config &cfg, const void *in, const void *bin, vo
       // 466-585) re-run it, with the reduced coefficient, for the patch groups whose previous pass
       // left an unphysical cell: every kernel returns at once for the others (`active`), and every
       // stage but the reconstruction gives the same values again
-      auto pass = [&]( const CtuArgs<R> &a )
+      const bool slices = !mm && !rp && !cfg.char_reconstruction && sizeof(R) == 4;
+      auto pass = [&]( const CtuArgs<R> &a ) -> cudaError_t
       {
          if ( mppm ) ctu_con2pri<R,P,MNX + 2><<< ctu_grid( NX3, n, B ), B, 0, st >>>( a );
          else if ( mm ) ctu_con2pri<R,P,MNX><<< ctu_grid( MNX3, n, B ), B, 0, st >>>( a );
@@ -1233,12 +1332,26 @@ int ctu_solve_t( const gb_fluid_config &cfg, const void *in, const void *bin, vo
          }
          else if ( rp && ppm ) rp_half_step<R,P,LR_PPM>( a, cfg.char_reconstruction, n, st );
          else if ( rp )  rp_half_step<R,P,LR_PLM>( a, cfg.char_reconstruction, n, st );
-         else if ( ppm ) ctu_half_step<R,P,LR_PPM>( a, cfg.char_reconstruction, n, st );
-         else            ctu_half_step<R,P,LR_PLM>( a, cfg.char_reconstruction, n, st );
-         if      ( mppm ) ctu_full_step<R,P,NX>( af, n, st );
-         else if ( mm )  ctu_full_step<R,P,MNX>( af, n, st );
-         else if ( ppm ) ctu_full_step<R,P,NX + 2>( af, n, st );
-         else            ctu_full_step<R,P,NX>( af, n, st );
+         else if ( !slices )
+         {
+            if ( ppm ) ctu_half_step<R,P,LR_PPM>( a, cfg.char_reconstruction, n, st );
+            else       ctu_half_step<R,P,LR_PLM>( a, cfg.char_reconstruction, n, st );
+         }
+         else if constexpr ( sizeof(R) == 4 )
+         {
+            const bool gmm = ( a.limiter == GB_LIM_GMINMOD && a.coeff < R(2) );
+            const cudaError_t e = ppm ? ( gmm ? ctu_slice_step<R,P,LR_PPM,true>( a, n, st ) : ctu_slice_step<R,P,LR_PPM,false>( a, n, st ) )
+                                      : ( gmm ? ctu_slice_step<R,P,LR_PLM,true>( a, n, st ) : ctu_slice_step<R,P,LR_PLM,false>( a, n, st ) );
+            if ( e != cudaSuccess ) return e;
+            af.fcf = a.fcv;
+            af.fcf_pg = 6*NM*NF3;
+         }
+         const bool flux = !slices;
+         if      ( mppm ) ctu_full_step<R,P,NX>( af, n, flux, st );
+         else if ( mm )  ctu_full_step<R,P,MNX>( af, n, flux, st );
+         else if ( ppm ) ctu_full_step<R,P,NX + 2>( af, n, flux, st );
+         else            ctu_full_step<R,P,NX>( af, n, flux, st );
+         return cudaSuccess;
       };
       const int maxit = ( mm || rp ) ? prm->minmod_maxiter : 0;
       int *flags = nullptr;
@@ -1248,7 +1361,7 @@ int ctu_solve_t( const gb_fluid_config &cfg, const void *in, const void *bin, vo
          if ( cudaMemsetAsync( flags, 0, 2*(size_t)n*sizeof(int), st ) != cudaSuccess ) return GB_E_CUDA;
          a.fail_next = flags;
       }
-      pass( a );
+      if ( pass( a ) != cudaSuccess ) return GB_E_CUDA;
       for (int it=1; it<=maxit; it++)
       {
          // AdaptiveMinModCoeff, in the precision of the reconstruction
@@ -1261,7 +1374,7 @@ int ctu_solve_t( const gb_fluid_config &cfg, const void *in, const void *bin, vo
          r.fail_next = ( it < maxit ) ? flags + (size_t)( it & 1 )*n : nullptr;
          if ( r.fail_next != nullptr && cudaMemsetAsync( r.fail_next, 0, (size_t)n*sizeof(int), st ) != cudaSuccess )
             return GB_E_CUDA;
-         pass( r );
+         if ( pass( r ) != cudaSuccess ) return GB_E_CUDA;
       }
       if ( cudaGetLastError() != cudaSuccess ) return GB_E_CUDA;
    }

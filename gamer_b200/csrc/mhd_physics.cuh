@@ -728,6 +728,25 @@ GB_DEV void mhd_eigen( const Phys<R> &ph, const R *w, R (&ev)[7], R (&LE)[7][7],
 }
 
 
+// y = A x: the Jacobian along D of the primitive equations (rho, v_n, v_t1, v_t2, P, B_t1, B_t2), whose
+// eigenvectors are mhd_eigen's, the normal field fixed.  A sound speed that is zero, infinite or not a
+// number leaves no eigenvectors: NaN, as from the wave sums.
+template <int D, typename R>
+GB_DEV void mhd_jacobian( const Phys<R> &ph, const R *w, const R (&x)[7], R (&y)[7] )
+{
+   typedef MDir<D> M;
+   const R rho = w[0], irho = R(1)/rho, gp = ph.gamma*w[4], a2 = gp*irho;
+   const R vn = ( a2 > R(0) && a2 <= Lim<R>::huge() ) ? w[M::n] : R(NAN);
+   const R Bn = w[M::bn], B1 = w[M::b1], B2 = w[M::b2];
+   y[0] = vn*x[0] + rho*x[1];
+   y[1] = vn*x[1] + irho*( x[4] + B1*x[5] + B2*x[6] );
+   y[2] = vn*x[2] - irho*Bn*x[5];
+   y[3] = vn*x[3] - irho*Bn*x[6];
+   y[4] = vn*x[4] + gp*x[1];
+   y[5] = vn*x[5] + B1*x[1] - Bn*x[2];
+   y[6] = vn*x[6] + B2*x[1] - Bn*x[3];
+}
+
 // MHD slopes limited in the 7-wave characteristic variables of the cell (Hydro_LimitSlope with MHD and
 // CHAR_RECONSTRUCTION, CPU_Shared_DataReconstruction.cpp:1918-2030, through Hydro_Pri2Char:1436-1486 and
 // Hydro_Char2Pri:1513-1576).  LE / RE are the cell's eigenvectors along D (mhd_eigen).  The normal B
