@@ -50,7 +50,7 @@ int ctu_solve( const gb_fluid_config &cfg, const void *flu_in, const void *mag_i
                void *flux, void *ele, int npg, const gb_fluid_params *prm, void *scratch, size_t scratch_bytes,
                cudaStream_t st );
 int mhm_rp_half( int precision, int rsolver, int nc, int nxi, const void *in, void *half, int npg, double dt, double dh,
-                 const Phys<double> &phd, cudaStream_t st );
+                 const Phys<double> &phd, int *status, cudaStream_t st );
 }
 
 namespace {
@@ -274,7 +274,7 @@ int solve_rp( gb_fluid_solver *s, const void *in, void *out, char *de, void *flu
       const int n = ( npg - p0 < chunk ) ? npg - p0 : chunk;
       const char *cin = (const char*)in + p0*bi;
       rc = gb::mhm_rp_half( s->cfg.precision, s->cfg.rsolver, s->ncomp, s->cfg.flu_nxt, cin, s->d_scratch[slot], n, dt, dh,
-                            phd, st );
+                            phd, s->d_status, st );
       if ( rc != GB_OK ) return rc;
       char *cout = (char*)out + p0*bo, *cde = de ? de + p0*bd : nullptr;
       void *cflux = flux ? (char*)flux + p0*bf : nullptr;

@@ -76,18 +76,12 @@ GB_DEV void con2pri_cc_pair( const Phys<float> &ph, const float2 *u, float2 *w )
 // HLLC with the left and right states' speeds formed as float2 lanes (x = left, y = right);
 // the star state and the upwind flux are the scalar riemann_hllc's
 // (CPU_Shared_RiemannSolver_HLLC.cpp:392-655, HD version)
-template <int D, int P, int NC>
-GB_DEV void riemann_hllc_pair( const Phys<float> &ph, const float *L, const float *Rt, float *fo )
+// ir, pp, cs: reciprocal density, pressure and sound speed of the two states
+template <int D, int NC>
+GB_DEV void hllc_pair_core( const Phys<float> &ph, const float *L, const float *Rt, float2 ir, float2 pp, float2 cs, float *fo )
 {
-   constexpr int n = Dir<D>::n, t1 = Dir<D>::t1, t2 = Dir<D>::t2;
-   const float2 dd = make_float2( L[0], Rt[0] );
-   const float2 ir = make_float2( 1.f/L[0], 1.f/Rt[0] );
-   const float2 mn = make_float2( L[n], Rt[n] );
-   const float2 uu = p_mul( ir, mn );
-   const float2 pp = pres_con_pair<P>( ph, dd, ir, mn, make_float2( L[t1], Rt[t1] ), make_float2( L[t2], Rt[t2] ),
-                                       make_float2( L[4], Rt[4] ) );
-   const float2 c2 = p_mul( p_mul( p_bc( ph.gamma ), pp ), ir );
-   const float2 cs = make_float2( sqrtf( c2.x ), sqrtf( c2.y ) );
+   constexpr int n = Dir<D>::n;
+   const float2 uu = p_mul( ir, make_float2( L[n], Rt[n] ) );
    const float2 wm = p_sub( uu, cs );            // (ul - csl, ur - csr)
    const float2 wp = p_add( uu, cs );            // (ul + csl, ur + csr)
    const float ul = uu.x, ur = uu.y, csl = cs.x, csr = cs.y, pl = pp.x, pr = pp.y;
@@ -120,21 +114,27 @@ GB_DEV void riemann_hllc_pair( const Phys<float> &ph, const float *L, const floa
    passive_upwind<NC>( fo, L, Rt, ir.x, ir.y );
 }
 
+template <int D, int P, int NC>
+GB_DEV void riemann_hllc_pair( const Phys<float> &ph, const float *L, const float *Rt, float *fo )
+{
+   constexpr int n = Dir<D>::n, t1 = Dir<D>::t1, t2 = Dir<D>::t2;
+   const float2 ir = make_float2( 1.f/L[0], 1.f/Rt[0] );
+   const float2 pp = pres_con_pair<P>( ph, make_float2( L[0], Rt[0] ), ir, make_float2( L[n], Rt[n] ),
+                                       make_float2( L[t1], Rt[t1] ), make_float2( L[t2], Rt[t2] ), make_float2( L[4], Rt[4] ) );
+   const float2 c2 = p_mul( p_mul( p_bc( ph.gamma ), pp ), ir );
+   hllc_pair_core<D,NC>( ph, L, Rt, ir, pp, make_float2( sqrtf( c2.x ), sqrtf( c2.y ) ), fo );
+}
+
 // Two HLLC problems as the lanes of float2 (e.g. an x face and a y face of the same plane), both
 // given in the rotated frame: 0 = density, 1 = normal momentum, 2 and 3 = the transverse momenta
 // in the order Hydro_Rotate3D gives them, 4 = energy.  Every lane follows riemann_hllc step by step
 // (CPU_Shared_RiemannSolver_HLLC.cpp:392-655, HD version); the upwind choice becomes a per-lane
 // select.  A lane whose flux comes out NaN is flagged in nan_x / nan_y for the HLLE rescue.
-template <int P>
-GB_DEV void riemann_hllc_x2( const Phys<float> &ph, const float2 (&L)[5], const float2 (&Rt)[5], float2 (&fo)[5],
-                             bool &nan_x, bool &nan_y )
+// irl, pl, csl (irr, pr, csr): reciprocal densities, pressures and sound speeds of the left (right) states.
+GB_DEV void hllc_x2_core( const Phys<float> &ph, const float2 (&L)[5], const float2 (&Rt)[5], float2 irl, float2 irr,
+                          float2 pl, float2 pr, float2 csl, float2 csr, float2 (&fo)[5], bool &nan_x, bool &nan_y )
 {
-   const float2 irl = make_float2( 1.f/L[0].x, 1.f/L[0].y ), irr = make_float2( 1.f/Rt[0].x, 1.f/Rt[0].y );
    const float2 ul = p_mul( irl, L[1] ), ur = p_mul( irr, Rt[1] );
-   const float2 pl = pres_con_pair<P>( ph, L[0],  irl, L[1],  L[2],  L[3],  L[4]  );
-   const float2 pr = pres_con_pair<P>( ph, Rt[0], irr, Rt[1], Rt[2], Rt[3], Rt[4] );
-   const float2 cl2 = p_mul( p_mul( p_bc( ph.gamma ), pl ), irl ), cr2 = p_mul( p_mul( p_bc( ph.gamma ), pr ), irr );
-   const float2 csl = make_float2( sqrtf( cl2.x ), sqrtf( cl2.y ) ), csr = make_float2( sqrtf( cr2.x ), sqrtf( cr2.y ) );
    const float2 wl1 = p_sub( ul, csl ), wl2 = p_sub( ur, csr ), wr1 = p_add( ul, csl ), wr2 = p_add( ur, csr );
    const float2 wl = make_float2( fminf( wl1.x, wl2.x ), fminf( wl1.y, wl2.y ) );
    const float2 wr = make_float2( fmaxf( wr1.x, wr2.x ), fmaxf( wr1.y, wr2.y ) );
@@ -188,7 +188,19 @@ GB_DEV void riemann_hllc_x2( const Phys<float> &ph, const float2 (&L)[5], const 
    for (int v=0; v<5; v++) { nan_x |= ( fo[v].x != fo[v].x );  nan_y |= ( fo[v].y != fo[v].y ); }
 }
 
-// PLM face states of both faces along D, primitive -> conserved, and the Hancock flux difference
+template <int P>
+GB_DEV void riemann_hllc_x2( const Phys<float> &ph, const float2 (&L)[5], const float2 (&Rt)[5], float2 (&fo)[5],
+                             bool &nan_x, bool &nan_y )
+{
+   const float2 irl = make_float2( 1.f/L[0].x, 1.f/L[0].y ), irr = make_float2( 1.f/Rt[0].x, 1.f/Rt[0].y );
+   const float2 pl = pres_con_pair<P>( ph, L[0],  irl, L[1],  L[2],  L[3],  L[4]  );
+   const float2 pr = pres_con_pair<P>( ph, Rt[0], irr, Rt[1], Rt[2], Rt[3], Rt[4] );
+   const float2 cl2 = p_mul( p_mul( p_bc( ph.gamma ), pl ), irl ), cr2 = p_mul( p_mul( p_bc( ph.gamma ), pr ), irr );
+   hllc_x2_core( ph, L, Rt, irl, irr, pl, pr, make_float2( sqrtf( cl2.x ), sqrtf( cl2.y ) ), make_float2( sqrtf( cr2.x ), sqrtf( cr2.y ) ),
+                 fo, nan_x, nan_y );
+}
+
+// PLM or PPM face states of both faces along D, primitive -> conserved, and the Hancock flux difference
 // (the float2 counterpart of recon_dir; fc[D][v] = (left face, right face) of variable v); CHARR:
 // PLM with CHAR_RECONSTRUCTION
 template <int D, int P, int NC, bool CHARR, bool HANC = true>

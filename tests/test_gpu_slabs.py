@@ -1,0 +1,105 @@
+"""Patch groups solved in slabs along z (the last, partly filled wave of a call) equal the same patch
+groups solved whole, bit for bit: a call that reports failed patch groups keeps them whole."""
+import numpy as np
+import pytest
+
+from gamer_b200 import ic
+from gamer_b200.fluid import FluidSolver, SolverParams
+
+pytestmark = pytest.mark.gpu
+GAMMA = 5.0 / 3.0
+
+
+def _windows(npg, nxt, dtype, dual=False):
+    box = ic.lognormal_box(4, seed=npg + nxt, gamma=GAMMA, dual=dual)
+    x = ic.cut_patch_groups(box, nxt).astype(dtype)
+    dh = 1.0 / 64
+    return np.concatenate([x] * (-(-npg // x.shape[0])))[:npg], ic.cfl_dt(box, GAMMA, dh, cfl=0.4), dh
+
+
+@pytest.mark.parametrize("npg", [1, 3, 8, 37, 64, 148, 297, 350])
+@pytest.mark.parametrize("kw,nxt", [
+    (dict(precision="fp32"), 20), (dict(precision="fp32", rsolver="roe"), 22), (dict(precision="mixed", lr="ppm", rsolver="roe"), 22),
+    (dict(precision="fp64"), 20), (dict(precision="fp64", lr="ppm"), 24), (dict(precision="fp32", dual_energy=True), 20),
+    (dict(scheme="mhm_rp", precision="mixed"), 22), (dict(scheme="mhm_rp", precision="fp64"), 22)])
+def test_slabs_equal_whole_patch_groups(cuda_device, npg, kw, nxt):
+    import torch
+    s = FluidSolver(gamma=GAMMA, flu_nxt=nxt, **kw)
+    x, dt, dh = _windows(npg, nxt, s.np_dtype, s.dual)
+    t = torch.from_numpy(x).cuda()
+    prm = SolverParams(dt=dt, dh=dh)
+    got = []
+    for report in (True, False):
+        out = torch.full((npg, s.ncomp, 16, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        flux = torch.full((npg, 9, s.ncomp, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        de = torch.full((npg, 16, 16, 16), 48, dtype=torch.int8, device="cuda") if s.dual else None
+        fail = torch.full((npg,), 7, dtype=torch.int32, device="cuda") if report else None
+        s.solve_device(t, out, prm, flux=flux, de_out=de, pg_fail=fail)
+        torch.cuda.synchronize()
+        assert s.status() == 0
+        assert fail is None or not bool(fail.any())
+        got.append((out, flux, de))
+    for a, b in zip(*got):
+        assert a is None or torch.equal(a, b)
+    assert bool(torch.isfinite(got[0][0]).all()) and bool(torch.isfinite(got[0][1]).all())
+
+
+@pytest.mark.parametrize("npg", [5, 300])
+def test_unphysical_cells_are_reported_from_slabs(cuda_device, npg):
+    """A patch group with a cell that ends up unphysical sets the status bit, whole or in slabs."""
+    import torch
+    s = FluidSolver(gamma=GAMMA, precision="fp32")
+    x, dt, dh = _windows(npg, 20, np.float32)
+    x[npg - 1, 4, 15, 9, 9] = 1.0e-3 * x[npg - 1, 4, 15, 9, 9]          # total energy below the kinetic one
+    t = torch.from_numpy(x).cuda()
+    out = torch.empty((npg, 5, 16, 16, 16), dtype=t.dtype, device="cuda")
+    fail = torch.zeros(npg, dtype=torch.int32, device="cuda")
+    s.solve_device(t, out, SolverParams(dt=dt, dh=dh, StoreFlux=False), pg_fail=fail)
+    torch.cuda.synchronize()
+    whole = s.status()
+    s.solve_device(t, out, SolverParams(dt=dt, dh=dh, StoreFlux=False))
+    torch.cuda.synchronize()
+    assert s.status() == whole and (whole != 0) == bool(fail.any())
+
+
+@pytest.mark.parametrize("lr,nxt", [("plm", 22), ("ppm", 24)])
+@pytest.mark.parametrize("prec", ["fp32", "mixed"])
+@pytest.mark.parametrize("npg", [1, 9, 148, 333])
+def test_mhm_rp_float_half_step_against_fp64(cuda_device, lr, nxt, prec, npg):
+    """The float half step with per-cell pressures and sound speeds against the FP64 solver (another
+    kernel) on the same float-rounded input."""
+    import torch
+    x, dt, dh = _windows(npg, nxt, np.float32)
+    got = []
+    for p in (prec, "fp64"):
+        s = FluidSolver(scheme="mhm_rp", lr=lr, precision=p, gamma=GAMMA)
+        t = torch.from_numpy(x.astype(s.np_dtype)).cuda()
+        out = torch.full((npg, 5, 16, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        flux = torch.full((npg, 9, 5, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        s.solve_device(t, out, SolverParams(dt=dt, dh=dh), flux=flux)
+        torch.cuda.synchronize()
+        assert s.status() == 0
+        got.append((out.double(), flux.double()))
+    for g, r in zip(*got):
+        v = 1 if g.dim() == 5 and g.shape[1] == 5 else 2
+        rms = (r * r).mean(dim=[d for d in range(g.dim()) if d != v], keepdim=True).sqrt()
+        # float rounding of a two-step scheme (a few dozen operations on each path), and the share of
+        # cells that take another limiter branch
+        err = (g - r).abs() / (r.abs() + rms)
+        assert float((err > 64 * 2.0 ** -23).double().mean()) < 1e-3
+        assert float(err.max()) < 5e-3
+
+
+@pytest.mark.parametrize("prec,npg,offset", [("fp32", 1, 0), ("fp32", 19, 0), ("fp32", 296, 0), ("fp32", 301, 0), ("fp32", 300, 1), ("mixed", 297, 0), ("fp64", 296, 0), ("fp64", 299, 1)])
+def test_dt_of_solver_outputs_equals_dt_of_patches(cuda_device, prec, npg, offset):
+    """One CTA per patch group (outputs, 16-byte aligned) against one per patch (patch arrays)."""
+    import torch
+    s = FluidSolver(precision=prec, gamma=GAMMA)
+    x, _, dh = _windows(npg, 16, s.np_dtype)
+    flat = torch.zeros(x.size + offset, dtype=s.torch_dtype, device="cuda")
+    flat[offset:] = torch.from_numpy(x.reshape(-1)).cuda()
+    got = s.dt_cfl(flat[offset:].view(x.shape), dh, from_output=True)
+    flu, _ = ic.patches_from_output(x)
+    ref = s.dt_cfl(torch.from_numpy(np.ascontiguousarray(flu)).cuda(), dh)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
