@@ -202,15 +202,15 @@ GB_DEV void riemann_hllc_x2( const Phys<float> &ph, const float2 (&L)[5], const 
 
 // PLM or PPM face states of both faces along D, primitive -> conserved, and the Hancock flux difference
 // (the float2 counterpart of recon_dir; fc[D][v] = (left face, right face) of variable v); CHARR:
-// PLM with CHAR_RECONSTRUCTION
-template <int D, int P, int NC, bool CHARR, bool HANC = true>
+// PLM with CHAR_RECONSTRUCTION; sl / sc / sr: the limited slopes of the three cells (PPM)
+template <int D, int P, int NC, bool CHARR, bool HANC = true, int LR = LR_PLM>
 GB_DEV void recon_dir_pair( const Phys<float> &ph, const float *cc, const float *pl, const float *pr,
                             int lim, float coeff, bool clamp, float2 (&fc)[3][NC], float (&fpres)[6],
-                            float (&acc)[NC] )
+                            float (&acc)[NC], const float *sl = nullptr, const float *sc = nullptr, const float *sr = nullptr )
 {
    constexpr int n = Dir<D>::n, t1 = Dir<D>::t1, t2 = Dir<D>::t2;
    float2 w[NC];
-   if constexpr ( CHARR )
+   if constexpr ( CHARR && LR == LR_PLM )
    {
       float fl[NC], fr[NC];
       plm_faces_char<D,NC>( ph, pl, cc, pr, lim, coeff, fl, fr );
@@ -223,7 +223,8 @@ GB_DEV void recon_dir_pair( const Phys<float> &ph, const float *cc, const float 
       for (int v=0; v<NC; v++)
       {
          float fl, fr;
-         plm_faces( pl[v], cc[v], pr[v], lim, coeff, clamp, fl, fr );
+         if constexpr ( LR == LR_PLM ) plm_faces( pl[v], cc[v], pr[v], lim, coeff, clamp, fl, fr );
+         else                          ppm_faces( pl[v], cc[v], pr[v], sl[v], sc[v], sr[v], lim, fl, fr );
          w[v] = make_float2( fl, fr );
       }
    }

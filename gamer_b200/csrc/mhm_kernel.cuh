@@ -243,11 +243,13 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
    constexpr bool LEAN = mhm_lean( sizeof(R), LR );   // PPM: slopes formed in place
    constexpr int AHEAD = LEAN ? 1 : ( CONV_A ? 3 : 2 );   // prefetch distance of the plane ring
    constexpr int LAG   = ( LR == LR_PPM ) ? 2 : 1;    // fc plane kf = t - NG - LAG at step t
-   // float PLM: the two faces of each direction are evaluated as one float2 (hydro_pair.cuh)
-   constexpr bool PAIR = std::is_same<R, float>::value && LR == LR_PLM;
+   // float: the two faces of each direction are evaluated as one float2 (hydro_pair.cuh); PPM with HLLC, 592
+   // patch groups: 294 -> 283 us, mixed with Roe, 1000: 691 -> 608
+   constexpr bool PAIR = std::is_same<R, float>::value;
    constexpr bool CARRY_SMEM = mhm_carry_smem( P, NC );   // per-column z state in shared memory
-   // float PLM HLLC without passive scalars: an x face and a y face per thread as float2 lanes
-   constexpr bool X2 = PAIR && RS == RS_HLLC && NC == 5;
+   // float HLLC without user passive scalars: an x face and a y face per thread as float2 lanes (the
+   // dual-energy field is then upwinded per lane; PPM, 592 patch groups: 373 -> 357 us)
+   constexpr bool X2 = PAIR && RS == RS_HLLC && NC <= 6;
    constexpr bool CHARR = ( LIMK == LIMK_CHAR );
    constexpr bool DUAL  = mhm_has_dual( NC );         // the last variable is the dual-energy field
    constexpr int  NPU   = NC - 5 - ( DUAL ? 1 : 0 );  // user passive scalars
@@ -314,10 +316,11 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
       const R dt = a.dt[lv], dh = a.dh[lv];
       const R dt_dh2 = R(0.5)*dt/dh;
       const A dt_dh  = (A)dt/(A)dh;
-      const R *g_in = a.in + (size_t)pg*NC*nin*nin2;
-      R *g_out = a.out + (size_t)pg*NC*PS2*PS2*PS2;
+      // (the input and the output from the slab's first plane on)
+      const R *g_in = a.in + (size_t)pg*NC*nin*nin2 + (size_t)o0*nin2;
+      R *g_out = a.out + (size_t)pg*NC*PS2*PS2*PS2 + o0*PS2*PS2;
       R *g_flux = ( a.flux != nullptr ) ? a.flux + (size_t)pg*9*NC*PS2*PS2 : nullptr;
-      char *g_de = ( a.de != nullptr ) ? a.de + (size_t)pg*PS2*PS2*PS2 : nullptr;
+      char *g_de = ( a.de != nullptr ) ? a.de + (size_t)pg*PS2*PS2*PS2 + o0*PS2*PS2 : nullptr;
 
       // one thread issues the bulk copies of cc plane c (all NC variables) into its ring slot
       auto issue = [&]( int c ) {
@@ -325,7 +328,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
          fence_proxy_async();
          mbar_expect_tx( &bar[q], plane_bytes );
          for (int v=0; v<NC; v++)
-            bulk_g2s( s_pln + ( q*NC + v )*nin2, g_in + (size_t)v*nin*nin2 + (size_t)( c + o0 + sh )*nin2,
+            bulk_g2s( s_pln + ( q*NC + v )*nin2, g_in + (size_t)v*nin*nin2 + (size_t)( c + sh )*nin2,
                       nin2*sizeof(R), &bar[q] );
       };
 
@@ -423,13 +426,52 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                      else               { i = 1 + r;   j = NFC - 1; }
                   }
                   const int ce = ( j + NG )*nin + ( i + NG );
-                  const size_t gidx = (size_t)( cz + o0 + sh )*nin2 + ( j + NG + sh )*nin + ( i + NG + sh );
+                  const size_t gidx = (size_t)( cz + sh )*nin2 + ( j + NG + sh )*nin + ( i + NG + sh );
                   R cc[NC], nl[NC], nr[NC];
                   R fcon[6][NC], fpres[6], acc[NC];
                   bool reset;
 #                 pragma unroll
                   for (int v=0; v<NC; v++) cc[v] = pc[v*nin2 + ce];
-                  if constexpr ( PAIR )
+                  if constexpr ( PAIR && LEAN )
+                  {
+                     float2 fc2[3][NC];
+                     // the neighbours along one direction (at ql and qr, two cells away qll and qrr) and the
+                     // limited slopes of the three cells
+                     R sl[NC], sc[NC], sr[NC];
+                     auto along = [&]( auto dir, const R *qll, const R *ql, const R *qr, const R *qrr )
+                     {
+                        constexpr int D = decltype( dir )::value;
+                        if constexpr ( CHARR )
+                        {
+                           R ll[NC], rr[NC];
+#                          pragma unroll
+                           for (int v=0; v<NC; v++) { nl[v] = ql[v*nin2];  nr[v] = qr[v*nin2];  ll[v] = qll[v*nin2];  rr[v] = qrr[v*nin2]; }
+                           ppm_char_slopes<D,NC>( ph, ll, nl, cc, nr, rr, lim, coeff, sl, sc, sr );
+                        }
+                        else
+                        {
+#                          pragma unroll
+                           for (int v=0; v<NC; v++)
+                           {
+                              nl[v] = ql[v*nin2];  nr[v] = qr[v*nin2];
+                              sl[v] = limit_slope( qll[v*nin2], nl[v], cc[v], lim, coeff );
+                              sc[v] = limit_slope( nl[v], cc[v], nr[v], lim, coeff );
+                              sr[v] = limit_slope( cc[v], nr[v], qrr[v*nin2], lim, coeff );
+                           }
+                        }
+                        recon_dir_pair<D,P,NC,CHARR,!RP,LR_PPM>( ph, cc, nl, nr, lim, coeff, clamp, fc2, fpres, acc, sl, sc, sr );
+                     };
+                     const R *q0 = pc + ce;
+                     along( std::integral_constant<int,0>(), q0 - 2, q0 - 1, q0 + 1, q0 + 2 );
+                     along( std::integral_constant<int,1>(), q0 - 2*nin, q0 - nin, q0 + nin, q0 + 2*nin );
+                     along( std::integral_constant<int,2>(), plane( cz - 2 ) + ce, pm + ce, pp + ce, plane( cz + 2 ) + ce );
+                     if constexpr ( !RP ) hancock_finish_pair<P,NC>( ph, dt_dh2, fc2, fpres, acc, g_in + gidx, (size_t)nin*nin2, reset );
+#                    pragma unroll
+                     for (int d=0; d<3; d++)
+#                       pragma unroll
+                        for (int v=0; v<NC; v++) { fcon[2*d][v] = fc2[d][v].x;  fcon[2*d+1][v] = fc2[d][v].y; }
+                  }
+                  else if constexpr ( PAIR )
                   {
                      float2 fc2[3][NC];
 #                    pragma unroll
@@ -549,12 +591,12 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                         if ( kf >= 2 )
                         {
                            // output plane o = kf-2: its x/y fluxes are those of fc plane kf-1
-                           const int o = o0 + kf - 2, oi0 = i - 1, oj0 = j - 1;
+                           const int o = kf - 2, oi0 = i - 1, oj0 = j - 1;
                            const FP *fx = s_flx, *fy = s_fly;
                            // U_in of the output cell: the input at offset FLU_GHOST_SIZE (MHM_RP: the
                            // conserved 22^3 input, FLU_GHOST_SIZE = 3)
                            constexpr size_t ustride = RP ? (size_t)RPX*RPX*RPX : (size_t)nin*nin2;
-                           const R *uin = RP ? a.uin + (size_t)pg*NC*ustride + (size_t)( o + RPG )*RPX*RPX + ( oj0 + RPG )*RPX + ( oi0 + RPG )
+                           const R *uin = RP ? a.uin + (size_t)pg*NC*ustride + (size_t)( o0 + o + RPG )*RPX*RPX + ( oj0 + RPG )*RPX + ( oi0 + RPG )
                                              : g_in + (size_t)( o + G + sh )*nin2 + ( oj0 + G + sh )*nin + ( oi0 + G + sh );
                            R u[NC];
 #                          pragma unroll
@@ -638,24 +680,32 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                      }
                      bool nan_x, nan_y;
                      riemann_hllc_x2<P>( ph, L, Rr, F, nan_x, nan_y );
-                     float Fx[5], Fy[5];
+                     float Fx[NC], Fy[NC];
 #                    pragma unroll
                      for (int q=0; q<5; q++) { Fx[q] = F[q].x;  Fy[ry[q]] = F[q].y; }
                      if ( nan_x || nan_y )
+                     if constexpr ( NC > 5 )
+                     {
+                        // the dual-energy field with the mass flux (passive_upwind per lane)
+                        const bool ux = ( F[0].x >= 0.f ), uy = ( F[0].y >= 0.f );
+                        Fx[5] = s_fcx[( ( ux ? NC : 0 ) + 5 )*PS2*NFC + ox + ( ux ? 0 : 1 )]*( F[0].x*( 1.f/( ux ? L[0].x : Rr[0].x ) ) );
+                        Fy[5] = s_fcy[( ( uy ? NC : 0 ) + 5 )*NFC*PS2 + oy + ( uy ? 0 : PS2 )]*( F[0].y*( 1.f/( uy ? L[0].y : Rr[0].y ) ) );
+                        nan_x |= ( Fx[5] != Fx[5] );  nan_y |= ( Fy[5] != Fy[5] );
+                     }
                      {
                         // HLLE rescue of a NaN flux (CPU_Shared_ComputeFlux.cpp:313-362), per face
-                        float l[5], r[5];
+                        float l[NC], r[NC];
                         if ( nan_x )
                         {
 #                          pragma unroll
-                           for (int q=0; q<5; q++) { l[q] = L[q].x;  r[q] = Rr[q].x; }
-                           riemann_hlle_outlined<0,P,5>( ph, l, r, Fx );
+                           for (int v=0; v<NC; v++) { l[v] = s_fcx[( NC + v )*PS2*NFC + ox];  r[v] = s_fcx[v*PS2*NFC + ox + 1]; }
+                           riemann_hlle_outlined<0,P,NC>( ph, l, r, Fx );
                         }
                         if ( nan_y )
                         {
 #                          pragma unroll
-                           for (int q=0; q<5; q++) { l[ry[q]] = L[q].y;  r[ry[q]] = Rr[q].y; }
-                           riemann_hlle_outlined<1,P,5>( ph, l, r, Fy );
+                           for (int v=0; v<NC; v++) { l[v] = s_fcy[( NC + v )*NFC*PS2 + oy];  r[v] = s_fcy[v*NFC*PS2 + oy + PS2]; }
+                           riemann_hlle_outlined<1,P,NC>( ph, l, r, Fy );
                         }
                      }
 #                    pragma unroll
