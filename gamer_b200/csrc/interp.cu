@@ -24,6 +24,7 @@
 // bit for bit (in FP64 always; in FP32 as long as no intermediate is subnormal -- the device flushes
 // those to zero).
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 #include "../../include/gamer_b200_fluid.h"
 #include "gb_common.cuh"
@@ -379,7 +380,7 @@ __device__ __noinline__ void iterate_parent( const IntArgs<R> &a, const R *cb, s
 // from global memory).  The children of the five variables stay in registers: with a run-time loop
 // over the variables they went through local memory.  Bound by the issue of the 19 one-dimensional
 // operators of a parent's variable, each of rounded multiplications and selects.  With the assembly
-// below, 342 windows of 20^3, FP32: 217 -> 97 us (the bytes of both alone: 27 us).
+// below, 342 windows of 20^3, FP32: 217 -> 85 us (the bytes of both alone: 27 us).
 constexpr int INT_THREADS = 256;
 
 // CTAs per SM: 342 regions of 12^3 cells, with the window assembly, us: FP32 1: 137, 2: 111, 3: 97, 4: 103
@@ -450,13 +451,15 @@ __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_k
 }
 
 // planes of parents per CTA and their shared memory: half the parents' planes, fewer where those need
-// more than 48 KB (four CTAs share an SM), one at least; 0 bytes where even that needs over 200 KB
+// more than 48 KB (four CTAs share an SM) or where few regions would leave SMs idle, one at least;
+// 0 bytes where even that needs over 200 KB
 template <typename R>
 int interp_depth( int scheme, const IntArgs<R> &a, size_t *smem )
 {
    const int G = int_ghost( scheme );
    const size_t plane = (size_t)5*a.csize[0]*a.csize[1]*sizeof(R);
    int depth = ( a.crange[2] + 1 )/2;
+   while ( depth > 1 && (long long)a.nbatch*( ( a.crange[2] + depth - 1 )/depth ) < 296 ) depth = ( depth + 1 )/2;
    while ( depth > 1 && ( depth + 2*G )*plane > 48*1024 ) depth--;
    *smem = ( depth + 2*G )*plane;
    if ( *smem > 200*1024 ) *smem = 0;
@@ -540,14 +543,16 @@ int interp_run( const gb_interp_params *p, const void *cdata, void *fdata, int n
 // group's own interior, the interior of the same-level patch group nbr[p][s], or the
 // coarse-interpolated window cint[p] (gb_interpolate_device over the window).
 //
-// One CTA fills the window of one variable of one patch group; the 27 sources are resolved once into
+// One CTA (of a few windows, several) fills the window of one variable of one patch group; the 27
+// sources are resolved once into
 // shared memory.  A thread writes four consecutive cells with 16-byte stores (VEC: a window is a
 // whole number of them, since its width is even; an array that is not 16-byte aligned takes scalar
 // stores).  NXT: the width, a constant for the usual ones, so that the index arithmetic divides by
-// constants.
+// constants.  PAIR: cells are read two at a time (an even ghost width, so that a pair lies in one side,
+// and sources aligned to a pair).
 constexpr int ASM_THREADS = 256;
 
-template <typename R, int NXT, bool VEC>
+template <typename R, int NXT, bool VEC, bool PAIR>
 __global__ void __launch_bounds__( ASM_THREADS ) assemble_windows_kernel( const R *fine, const int *nbr, const R *cint, R *win,
                                                                           int npg, int ncomp, int nxt_any )
 {
@@ -570,19 +575,27 @@ __global__ void __launch_bounds__( ASM_THREADS ) assemble_windows_kernel( const 
       __syncthreads();
       const R *ci = cint + (size_t)pv*n3;
       R *wo = win + (size_t)pv*n3;
-      for (int c0 = 4*threadIdx.x; c0 < n3; c0 += 4*ASM_THREADS)
+      for (int c0 = 4*( blockIdx.y*ASM_THREADS + threadIdx.x ); c0 < n3; c0 += 4*ASM_THREADS*gridDim.y)
       {
+         constexpr int S = PAIR ? 2 : 1;
          R val[4];
 #        pragma unroll
-         for (int q=0; q<4; q++)
+         for (int q=0; q<4; q += S)
          {
             const int c = c0 + q;
             const int k = c / n2, r = c - k*n2, j = r / nxt, i = r - j*nxt;
             const int x = i - g, y = j - g, z = k - g;
             const int dx = ( x < 0 ) ? -1 : ( x >= PS2 ), dy = ( y < 0 ) ? -1 : ( y >= PS2 ), dz = ( z < 0 ) ? -1 : ( z >= PS2 );
             const long long src = s_src[( dz + 1 )*9 + ( dy + 1 )*3 + ( dx + 1 )];
-            val[q] = ( src >= 0 ) ? fine[src + ( ( z - PS2*dz )*PS2 + ( y - PS2*dy ) )*PS2 + ( x - PS2*dx )]
-                                  : ( src == FROM_CINT ) ? ci[c] : R(NAN);
+            const R *from = ( src >= 0 ) ? fine + src + ( ( z - PS2*dz )*PS2 + ( y - PS2*dy ) )*PS2 + ( x - PS2*dx )
+                                         : ( src == FROM_CINT ) ? ci + c : nullptr;
+            if constexpr ( PAIR )
+            {
+               typedef typename std::conditional<sizeof(R) == 4, float2, double2>::type R2;
+               const R2 t = from ? *(const R2*)from : R2{ R(NAN), R(NAN) };
+               val[q] = t.x;  val[q+1] = t.y;
+            }
+            else val[q] = from ? *from : R(NAN);
          }
          if constexpr ( !VEC )
          {
@@ -599,14 +612,17 @@ template <typename R>
 int assemble_launch( const void *fine, const int *nbr, const void *cint, void *win, int npg, int ncomp, int nxt, cudaStream_t st )
 {
    const long long items = (long long)npg*ncomp;
-   const unsigned grid = (unsigned)( ( items < 0x7fffffffLL ) ? items : 0x7fffffffLL );
+   // few windows: several CTAs each, about four per SM in all
+   const dim3 grid( (unsigned)( ( items < 0x7fffffffLL ) ? items : 0x7fffffffLL ),
+                    (unsigned)( ( items >= 592 ) ? 1 : ( items <= 74 ) ? 8 : 592/items ) );
    const bool vec = ( (uintptr_t)win & 15u ) == 0;
-#  define GB_ASM( N, V ) assemble_windows_kernel<R,N,V><<< grid, ASM_THREADS, 0, st >>>( (const R*)fine, nbr, (const R*)cint, (R*)win, npg, ncomp, nxt )
-   if      ( !vec )      GB_ASM( 0, false );
-   else if ( nxt == 20 ) GB_ASM( 20, true );
-   else if ( nxt == 22 ) GB_ASM( 22, true );
-   else if ( nxt == 24 ) GB_ASM( 24, true );
-   else                  GB_ASM( 0, true );
+   const bool pair = ( ( (uintptr_t)fine | (uintptr_t)cint ) & ( 2*sizeof(R) - 1 ) ) == 0;
+#  define GB_ASM( N, V, P ) assemble_windows_kernel<R,N,V,P><<< grid, ASM_THREADS, 0, st >>>( (const R*)fine, nbr, (const R*)cint, (R*)win, npg, ncomp, nxt )
+   if      ( !vec )              GB_ASM( 0, false, false );
+   else if ( nxt == 20 && pair ) GB_ASM( 20, true, true );
+   else if ( nxt == 24 && pair ) GB_ASM( 24, true, true );
+   else if ( nxt == 22 )         GB_ASM( 22, true, false );
+   else                          GB_ASM( 0, true, false );
 #  undef GB_ASM
    return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
 }
