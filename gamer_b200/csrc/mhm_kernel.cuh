@@ -683,7 +683,6 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                      float Fx[NC], Fy[NC];
 #                    pragma unroll
                      for (int q=0; q<5; q++) { Fx[q] = F[q].x;  Fy[ry[q]] = F[q].y; }
-                     if ( nan_x || nan_y )
                      if constexpr ( NC > 5 )
                      {
                         // the dual-energy field with the mass flux (passive_upwind per lane)
@@ -692,6 +691,7 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                         Fy[5] = s_fcy[( ( uy ? NC : 0 ) + 5 )*NFC*PS2 + oy + ( uy ? 0 : PS2 )]*( F[0].y*( 1.f/( uy ? L[0].y : Rr[0].y ) ) );
                         nan_x |= ( Fx[5] != Fx[5] );  nan_y |= ( Fy[5] != Fy[5] );
                      }
+                     if ( nan_x || nan_y )
                      {
                         // HLLE rescue of a NaN flux (CPU_Shared_ComputeFlux.cpp:313-362), per face
                         float l[NC], r[NC];
