@@ -2,6 +2,7 @@
 // See adjoint.cuh for the derivation and the symbol names.
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include "../../include/gamer_b200_fluid.h"
 #include "adjoint.cuh"
 
@@ -563,6 +564,12 @@ __global__ void adj_con2pri_kernel( const __grid_constant__ AdjArgs<R> a )
    }
 }
 
+} // namespace gb
+
+#include "adjoint_fused.cuh"
+
+namespace gb {
+
 // ---- periodic box <-> patch-group windows ----------------------------------------------------
 // box layout [ncomp][Z][Y][X] (x fastest), X = 16*npx ...; patch group p = (pz*npy + py)*npx + px;
 // window [p][ncomp][nxt^3] with ghost width g = (nxt-16)/2 <= 16, wrapped periodically.
@@ -607,6 +614,32 @@ __global__ void box_gather_kernel( const R *box, R *win, int npx, int npy, int n
    }
 }
 
+// widths with an even ghost width and a multiple of four (20, 24): four consecutive cells of a window row per
+// thread, read in pairs (a pair never straddles the wrap: X is even, and so is the row's first x)
+// and written with one 16- (32-) byte store.  Sixteen steps of 1024 patch groups: 1528 -> 769 us
+template <typename R, int NXT>
+__global__ void __launch_bounds__( 256 ) box_gather4_kernel( const R *box, R *win, int npx, int npy, int npz, int nc )
+{
+   typedef typename std::conditional<sizeof(R) == 4, float2, double2>::type R2;
+   constexpr int G = ( NXT - PS2 )/2, C = NXT/4, N2 = NXT*NXT;
+   static_assert( NXT % 4 == 0 && G % 2 == 0, "rows of whole quadruples" );
+   const int w = blockIdx.x, p = w / nc, v = w - p*nc;
+   const int X = PS2*npx, Y = PS2*npy, Z = PS2*npz;
+   const int px = p % npx, py = ( p / npx ) % npy, pz = p / ( npx*npy );
+   const R *vol = box + (size_t)v*Z*( (size_t)Y*X );
+   R *out = win + (size_t)w*( NXT*N2 );
+   for (int e = threadIdx.x; e < C*NXT*NXT; e += 256)
+   {
+      const int i = 4*( e % C ), j = ( e / C ) % NXT, k = e / ( C*NXT );
+      const int y = wrap1( py*PS2 - G + j, Y ), z = wrap1( pz*PS2 - G + k, Z );
+      const R *row = vol + ( (size_t)z*Y + y )*X;
+      const R2 a = *(const R2*)( row + wrap1( px*PS2 - G + i, X ) ), b = *(const R2*)( row + wrap1( px*PS2 - G + i + 2, X ) );
+      R *o = out + k*N2 + j*NXT + i;
+      if constexpr ( sizeof(R) == 4 ) *(float4*)o = make_float4( a.x, a.y, b.x, b.y );
+      else { ( (R2*)o )[0] = a;  ( (R2*)o )[1] = b; }
+   }
+}
+
 template <typename R>
 __global__ void box_scatter_kernel( const R *out, R *box, int npx, int npy, int npz, int nc )
 {
@@ -615,6 +648,7 @@ __global__ void box_scatter_kernel( const R *out, R *box, int npx, int npy, int 
    if ( t >= X*Y ) return;
    const int v = blockIdx.z;
    const int x = t % X, y = t / X;
+#  pragma unroll 8
    for (int z = blockIdx.y*PS2; z < blockIdx.y*PS2 + PS2; z++)
    {
       const int p = ( ( z/PS2 )*npy + y/PS2 )*npx + x/PS2;
@@ -663,6 +697,52 @@ __global__ void box_gather_adjoint_kernel( const double *wbar, double *boxbar, i
    }
 }
 
+// ghost widths up to 8, where a coordinate has at most two images per axis (the second on one side
+// only): the eight candidate entries of a cell are loaded under predicates, all in flight at once,
+// and added in the order of box_gather_adjoint_kernel.  Sixteen steps of 1024 patch groups: 1243 -> 1131 us
+__global__ void __launch_bounds__( 256 ) box_gather_adjoint2_kernel( const double *wbar, double *boxbar, int npx, int npy, int npz, int nxt, int nc )
+{
+   const int X = PS2*npx, Y = PS2*npy, Z = PS2*npz;
+   const int t = blockIdx.x*blockDim.x + threadIdx.x;
+   if ( t >= X*Y ) return;
+   const int v = blockIdx.z;
+   const int x = t % X, y = t / X;
+   const int g = ( nxt - PS2 )/2, n3 = nxt*nxt*nxt;
+   int px[3], ix[3], py[3], iy[3];
+   const int nx = axis_images( x, npx, g, px, ix );
+   const int ny = axis_images( y, npy, g, py, iy );
+   if ( nx < 2 ) { px[1] = px[0];  ix[1] = ix[0]; }
+   if ( ny < 2 ) { py[1] = py[0];  iy[1] = iy[0]; }
+   const size_t sz = (size_t)npy*npx*nc*n3, sy = (size_t)npx*nc*n3, sx = (size_t)nc*n3;      // strides of a patch group
+   const double *base[2][2];
+#  pragma unroll
+   for (int b=0; b<2; b++)
+#     pragma unroll
+      for (int a=0; a<2; a++) base[b][a] = wbar + py[b]*sy + px[a]*sx + (size_t)v*n3 + iy[b]*nxt + ix[a];
+#  pragma unroll 2
+   for (int z = blockIdx.y*PS2; z < blockIdx.y*PS2 + PS2; z++)
+   {
+      int pz[3], iz[3];
+      const int nz = axis_images( z, npz, g, pz, iz );
+      if ( nz < 2 ) { pz[1] = pz[0];  iz[1] = iz[0]; }
+      double q[2][2][2];
+#     pragma unroll
+      for (int c=0; c<2; c++)
+#        pragma unroll
+         for (int b=0; b<2; b++)
+#           pragma unroll
+            for (int a=0; a<2; a++) q[c][b][a] = ( c < nz && b < ny && a < nx ) ? base[b][a][pz[c]*sz + (size_t)iz[c]*nxt*nxt] : 0.0;
+      double s = 0.0;
+#     pragma unroll
+      for (int c=0; c<2; c++)
+#        pragma unroll
+         for (int b=0; b<2; b++)
+#           pragma unroll
+            for (int a=0; a<2; a++) if ( c < nz && b < ny && a < nx ) s += q[c][b][a];
+      boxbar[( (size_t)v*Z + z )*( (size_t)Y*X ) + t] = s;
+   }
+}
+
 // adjoint of box_scatter_kernel (interiors): window outputs gather the box adjoint
 __global__ void box_scatter_adjoint_kernel( const double *boxbar, double *outbar, int npx, int npy, int npz, int nc )
 {
@@ -671,6 +751,7 @@ __global__ void box_scatter_adjoint_kernel( const double *boxbar, double *outbar
    if ( t >= X*Y ) return;
    const int v = blockIdx.z;
    const int x = t % X, y = t / X;
+#  pragma unroll 8
    for (int z = blockIdx.y*PS2; z < blockIdx.y*PS2 + PS2; z++)
    {
       const int p = ( ( z/PS2 )*npy + y/PS2 )*npx + x/PS2;
@@ -699,6 +780,42 @@ size_t adj_ws_bytes_pg( int rsize )
         + (size_t)( 3*ADJ_NC + 1 )*ADJ_F3            // tape + reset flags
         + (size_t)6*ADJ_NC*ADJ_F3*8                  // qbar
         + (size_t)2*ADJ_NC*ADJ_N3*8 + 256*6;         // wbar, uext, alignment slack
+}
+
+// The fused kernel costs a whole wave of one patch group per SM (0.227 ms) whatever it holds, the
+// separate kernels 2.2 us a patch group: two steps forward and back, us, separate -> fused: 64 patch groups
+// 685 -> 725, 100: 890 -> 778, 148: 1120 -> 809, 180: 1341 -> 1373, 300: 2073 -> 1929.  The line
+// lies where the waves are two thirds full (100 patch groups a wave of 148).
+bool adjoint_fused_pays( int npg )
+{
+   int dev = 0, nsm = 0;
+   if ( cudaGetDevice( &dev ) != cudaSuccess ||
+        cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev ) != cudaSuccess || nsm < 1 ) return false;
+   const long long waves = ( (long long)npg + nsm - 1 )/nsm;
+   return 3*(long long)npg >= 2*waves*nsm;
+}
+
+// the plane-streaming kernel over all npg patch groups (float, HLLC)
+int adjoint_fused( const gb_fluid_config &cfg, const void *flu_in, const double *gout, double *gin, int npg,
+                   const gb_fluid_params *prm, int *nan_pg, int *status, cudaStream_t st )
+{
+   AdjArgs<float> a;
+   memset( (void*)&a, 0, sizeof(a) );
+   a.in = (const float*)flu_in;  a.gout = gout;  a.gin = gin;  a.npg = npg;
+   a.coeff = (float)prm->minmod_coeff;
+   a.ph.gamma = (float)cfg.gamma;  a.ph.gm1 = (float)( cfg.gamma - 1.0 );  a.ph.inv_gm1 = (float)( 1.0/( cfg.gamma - 1.0 ) );
+   a.ph.min_dens = (float)prm->min_dens;  a.ph.min_pres = (float)prm->min_pres;  a.ph.min_eint = (float)prm->min_eint;
+   a.ph.de_switch = (float)prm->dual_energy_switch;
+   a.dt = (float)prm->dt;  a.dh = (float)prm->dh;
+   int dev = 0, nsm = 0;
+   cudaGetDevice( &dev );
+   cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
+   const int smem = AdjFusedSmem::bytes, grid = ( npg < nsm ) ? npg : nsm;
+   if ( cudaFuncSetAttribute( adj_fused_kernel<P_FP32,false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem ) != cudaSuccess ||
+        cudaFuncSetAttribute( adj_fused_kernel<P_FP32,true>,  cudaFuncAttributeMaxDynamicSharedMemorySize, smem ) != cudaSuccess ) return GB_E_CUDA;
+   adj_fused_kernel<P_FP32,false><<< grid, AF_THREADS, smem, st >>>( a, nan_pg, status );
+   adj_fused_kernel<P_FP32,true> <<< grid, AF_THREADS, smem, st >>>( a, nan_pg, status );
+   return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
 }
 
 template <typename R, int P>
@@ -767,6 +884,7 @@ bool adjoint_supported( const gb_fluid_config &c, const gb_fluid_params *p )
 // the solver handle's configuration is needed here: read it through the public creation record
 struct gb_fluid_solver;
 extern "C" int gb_fluid_get_config( const gb_fluid_solver *s, gb_fluid_config *cfg );
+namespace gb { int *solver_status( gb_fluid_solver *s ); }
 
 extern "C" {
 
@@ -788,6 +906,11 @@ int gb_fluid_adjoint_step_device( gb_fluid_solver *s, const void *flu_in, const 
    if ( flu_in == nullptr || gout == nullptr || gin == nullptr || workspace == nullptr ) return GB_E_INVALID;
    if ( !( prm->dh > 0.0 ) || !( prm->dt >= 0.0 ) ) return GB_E_INVALID;
    if ( !adjoint_supported( c, prm ) ) return GB_E_UNSUPPORTED;
+   // the bulk copies of flu_in and gout start on 16-byte boundaries; the workspace holds the flags
+   if ( c.precision == GB_PREC_FP32 && c.rsolver == GB_RSOLVER_HLLC &&
+        ( ( (uintptr_t)flu_in | (uintptr_t)gout ) & 15u ) == 0 && ( (uintptr_t)workspace & 3u ) == 0 &&
+        ws_bytes >= adj_ws_bytes_pg( 4 ) && ws_bytes >= (size_t)npg*sizeof(int) && adjoint_fused_pays( npg ) )
+      return adjoint_fused( c, flu_in, gout, gin, npg, prm, (int*)workspace, solver_status( s ), (cudaStream_t)stream );
    if ( c.precision == GB_PREC_FP64 )
       return adjoint_step_t<double,P_FP64>( c, flu_in, gout, gin, npg, prm, workspace, ws_bytes, (cudaStream_t)stream );
    return adjoint_step_t<float,P_FP32>( c, flu_in, gout, gin, npg, prm, workspace, ws_bytes, (cudaStream_t)stream );
@@ -804,7 +927,16 @@ int gb_box_gather_device( const void *box, void *windows, int npx, int npy, int 
    const dim3 grid( (unsigned)nwin );
    // compile-time widths: one thread per (i, j) column of a window; otherwise 256 threads over its cells
 #  define GB_GATHER( R, N ) box_gather_kernel<R,N><<< grid, ( N > 0 ) ? N*N : 256, 0, st >>>( (const R*)box, (R*)windows, npx, npy, npz, nxt, ncomp )
-   if ( precision == GB_PREC_FP64 )
+   // quadruples of cells where both arrays allow the wider accesses
+   const size_t rs = ( precision == GB_PREC_FP64 ) ? 8 : 4;
+   const bool quads = ( (uintptr_t)box & ( 2*rs - 1 ) ) == 0 && ( (uintptr_t)windows & 15u ) == 0;
+#  define GB_GATHER4( R, N ) box_gather4_kernel<R,N><<< grid, 256, 0, st >>>( (const R*)box, (R*)windows, npx, npy, npz, ncomp )
+   if ( quads && ( nxt == 20 || nxt == 24 ) )
+   {
+      if ( precision == GB_PREC_FP64 ) { if ( nxt == 20 ) GB_GATHER4( double, 20 ); else GB_GATHER4( double, 24 ); }
+      else                             { if ( nxt == 20 ) GB_GATHER4( float, 20 );  else GB_GATHER4( float, 24 ); }
+   }
+   else if ( precision == GB_PREC_FP64 )
    {
       if      ( nxt == 20 ) GB_GATHER( double, 20 );
       else if ( nxt == 22 ) GB_GATHER( double, 22 );
@@ -817,6 +949,7 @@ int gb_box_gather_device( const void *box, void *windows, int npx, int npy, int 
       else                  GB_GATHER( float, 0 );
    }
 #  undef GB_GATHER
+#  undef GB_GATHER4
    return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
 }
 
@@ -843,7 +976,8 @@ int gb_box_gather_adjoint_device( const double *wbar, double *boxbar, int npx, i
    long long nwin = 0, nplane = 0;
    if ( !box_dims_ok( npx, npy, npz, ncomp, &nwin, &nplane ) ) return GB_E_INVALID;
    const dim3 grid( (unsigned)( ( nplane + 255 )/256 ), npz, ncomp );
-   box_gather_adjoint_kernel<<< grid, 256, 0, (cudaStream_t)stream >>>( wbar, boxbar, npx, npy, npz, nxt, ncomp );
+   if ( ( nxt - PS2 )/2 <= PS1 ) box_gather_adjoint2_kernel<<< grid, 256, 0, (cudaStream_t)stream >>>( wbar, boxbar, npx, npy, npz, nxt, ncomp );
+   else                          box_gather_adjoint_kernel<<< grid, 256, 0, (cudaStream_t)stream >>>( wbar, boxbar, npx, npy, npz, nxt, ncomp );
    return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
 }
 

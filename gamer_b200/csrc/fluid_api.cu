@@ -36,6 +36,9 @@ struct gb_fluid_solver {
 };
 
 namespace gb {
+// the device status word of a solver, for the calls whose kernels live in other files
+int *solver_status( gb_fluid_solver *s ) { return s->d_status; }
+
 size_t ctu_scratch_bytes_per_pg( int precision );
 size_t mhmrp_mhd_scratch_bytes_per_pg( int precision );
 size_t mhmrp_ppm_mhd_scratch_bytes_per_pg( int precision );
