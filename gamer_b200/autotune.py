@@ -136,7 +136,7 @@ def tune(scheme="mhm", lr="plm", rsolver="hllc", precision="fp32", dual=False, f
         name = torch.cuda.get_device_name(dev)
         by = {}
         for n, (best, res) in found.items():
-            dflt = res.get((256 if precision == "fp64" else 320, 0, 0))     # the library's default launch
+            dflt = res.get((352 if precision == "fp64" else 320, 0, 0))     # the library's default launch
             by[str(n)] = {"block": best[0], "ctas": best[1], "reg": best[2], "ms": res[best],
                           "default_ms": dflt,
                           "all_ms": {f"{b}/{c}/{r}": v for (b, c, r), v in sorted(res.items())}}

@@ -60,10 +60,13 @@ namespace {
 
 // tuned launch shapes on B200 (gamer_b200/autotune.py, gamer_b200/tuned.json): the float kernels keep
 // 2 CTAs of 320 threads per SM (one face-state cell per thread per plane), with dual energy too
-// (mixed, 1000 patch groups: 320 -> 0.443 ms, 448 -> 0.588 ms) and for PPM; FP64 is bounded to 256
+// (mixed, 1000 patch groups: 320 -> 0.443 ms, 448 -> 0.588 ms) and for PPM; FP64 (one CTA per SM)
+// takes 352: 320 face-state cells in one round beside a warp that converts the next plane, and 544 x / y
+// faces in two rounds, where 256 threads take two and three (PLM HLLC, 512 patch groups: 256 threads at
+// 255 registers 527 us, 384 at 168 402; input in L2, at 168 registers 256: 472, 320: 363, 352: 361, 384: 364)
 int default_block( const gb_fluid_config &c )
 {
-   if ( c.precision == GB_PREC_FP64 ) return 256;
+   if ( c.precision == GB_PREC_FP64 ) return 352;
    return 320;
 }
 constexpr int GB_HOST_CHUNK    = 256;     // patch groups per pipelined chunk of gb_fluid_solve_host

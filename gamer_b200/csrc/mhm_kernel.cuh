@@ -121,7 +121,7 @@ __host__ __device__ constexpr bool mhm_has_dual( int nc ) { return nc == 6 || nc
 
 // the per-column z state (2*NC values) is kept in shared memory instead of registers by the mixed
 // policy (its double accumulation leaves no registers for it) and by the float kernels with user
-// passive scalars (96 registers); the FP64 kernels (255 registers) keep it in registers, which
+// passive scalars (96 registers); the FP64 kernels (168 registers) keep it in registers, which
 // leaves the shared memory to the planes (FP64 with 7 variables: 215 KB)
 __host__ __device__ constexpr bool mhm_carry_smem( int p, int nc ) { return p == P_MIXED || ( nc > 6 && p == P_FP32 ); }
 
@@ -224,10 +224,11 @@ constexpr int SCH_MHM = 0, SCH_MHM_RP = 1;
 constexpr int RP_NX = 22, RP_NV = 20;
 
 // Registers: the float kernels are held to 96 per thread, so that two CTAs of 320 threads (the
-// default launch) share an SM; FP64 (one CTA of 256 per SM) may use all 255.  REG != 0 caps them at
+// default launch) share an SM; FP64 (one CTA of up to 384 per SM: three warps on each quarter) may use 168.
+// FP64 PLM, 512 patch groups: 255 registers and 256 threads 526 us, 168 and 384: 398, 352: 395.  REG != 0 caps them at
 // REG instead (the autotuner's register variants: 64 / 72 / 80 let two CTAs of 512 / 448 / 384
 // threads share an SM, 128 two CTAs of 256).
-constexpr int mhm_maxnreg( int rsize, int reg ) { return reg ? reg : ( rsize == 8 ? 255 : 96 ); }
+constexpr int mhm_maxnreg( int rsize, int reg ) { return reg ? reg : ( rsize == 8 ? 168 : 96 ); }
 
 template <typename R, int P, int LR, int RS, int NC, int NIN, int LIMK, int SCH = SCH_MHM, int REG = 0>
 __global__ void __maxnreg__( mhm_maxnreg( (int)sizeof(R), REG ) )
