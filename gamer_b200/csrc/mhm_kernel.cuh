@@ -686,10 +686,10 @@ mhm_kernel( const __grid_constant__ MhmArgs<R> a )
                      for (int q=0; q<5; q++) { Fx[q] = F[q].x;  Fy[ry[q]] = F[q].y; }
                      if constexpr ( NC > 5 )
                      {
-                        // the dual-energy field with the mass flux (passive_upwind per lane)
+                        // the dual-energy field with the mass flux (passive_upwind per lane; the reciprocals are HLLC's)
                         const bool ux = ( F[0].x >= 0.f ), uy = ( F[0].y >= 0.f );
-                        Fx[5] = s_fcx[( ( ux ? NC : 0 ) + 5 )*PS2*NFC + ox + ( ux ? 0 : 1 )]*( F[0].x*( 1.f/( ux ? L[0].x : Rr[0].x ) ) );
-                        Fy[5] = s_fcy[( ( uy ? NC : 0 ) + 5 )*NFC*PS2 + oy + ( uy ? 0 : PS2 )]*( F[0].y*( 1.f/( uy ? L[0].y : Rr[0].y ) ) );
+                        Fx[5] = s_fcx[( ( ux ? NC : 0 ) + 5 )*PS2*NFC + ox + ( ux ? 0 : 1 )]*( F[0].x*( ux ? 1.f/L[0].x : 1.f/Rr[0].x ) );
+                        Fy[5] = s_fcy[( ( uy ? NC : 0 ) + 5 )*NFC*PS2 + oy + ( uy ? 0 : PS2 )]*( F[0].y*( uy ? 1.f/L[0].y : 1.f/Rr[0].y ) );
                         nan_x |= ( Fx[5] != Fx[5] );  nan_y |= ( Fy[5] != Fy[5] );
                      }
                      if ( nan_x || nan_y )
