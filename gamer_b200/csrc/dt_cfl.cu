@@ -11,6 +11,7 @@
 // patches of each patch group in GAMER's LocalID order (TABLE_02, src/Tables/Table_02.cpp), so the
 // next step's dt needs no host-side repacking.
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "../../include/gamer_b200_fluid.h"
 #include "hydro_physics.cuh"
 
@@ -130,17 +131,20 @@ __global__ void __launch_bounds__( DT_BLOCK ) dt_cfl_kernel( const R *flu, const
 }
 
 // the eight patches of one patch group of hydro solver outputs per CTA: each thread reads four
-// neighbouring cells of a variable with one 16- (32-) byte load, 64 threads a plane, so that a warp's rows
+// neighbouring cells of a variable with one 16-byte load, 64 threads a plane, so that a warp's rows
 // are whole 64-byte lines instead of the 32-byte halves of one patch.  Bound by DRAM (2048 patch groups,
 // FP32: 40.5 -> 36 us, the output alone 26 us).
 constexpr int DT_PG_BLOCK = 256;
 // fewer than two such CTAs per SM leave it idle, and one CTA per patch is faster: a closing pass of a few
 // FP64 patch groups (correction, flux fix-up, dt) took 39.0 us by patches, 41.6 by patch groups
+// (444 patch groups, FP32: 16.3 -> 14.4 us).  FP64 reads whole lines either way: 600 patch groups 29.5 us by
+// patches, 32.7 by patch groups, so it stays with the patches
 constexpr int DT_PG_MIN = 296;
 
-template <typename R, int P>
-__global__ void __launch_bounds__( DT_PG_BLOCK ) dt_cfl_pg_kernel( const R *flu, R *dt, int ncomp, Phys<R> ph, R dh_safety )
+template <int P>
+__global__ void __launch_bounds__( DT_PG_BLOCK ) dt_cfl_pg_kernel( const float *flu, float *dt, int ncomp, Phys<float> ph, float dh_safety )
 {
+   typedef float R;
    constexpr int V = PS2*PS2*PS2;
    const int tid = threadIdx.x, pg = blockIdx.x;
    const R *u = flu + (size_t)pg*ncomp*V;
@@ -153,16 +157,8 @@ __global__ void __launch_bounds__( DT_PG_BLOCK ) dt_cfl_pg_kernel( const R *flu,
 #     pragma unroll
       for (int v=0; v<5; v++)
       {
-         if constexpr ( sizeof(R) == 4 )
-         {
-            const float4 t = *(const float4*)( u + v*V + c );
-            q[v][0] = t.x;  q[v][1] = t.y;  q[v][2] = t.z;  q[v][3] = t.w;
-         }
-         else
-         {
-            const double2 t0 = ( (const double2*)( u + v*V + c ) )[0], t1 = ( (const double2*)( u + v*V + c ) )[1];
-            q[v][0] = t0.x;  q[v][1] = t0.y;  q[v][2] = t1.x;  q[v][3] = t1.y;
-         }
+         const float4 t = *(const float4*)( u + v*V + c );
+         q[v][0] = t.x;  q[v][1] = t.y;  q[v][2] = t.z;  q[v][3] = t.w;
       }
 #     pragma unroll
       for (int k=0; k<4; k++)
@@ -199,11 +195,17 @@ int launch_dt( const gb_fluid_config &c, const void *flu, const void *mag, void 
    ph.gamma = (R)c.gamma;  ph.gm1 = (R)( c.gamma - 1.0 );  ph.inv_gm1 = (R)( 1.0/( c.gamma - 1.0 ) );
    ph.min_dens = R(0);  ph.min_pres = (R)min_pres;  ph.min_eint = R(0);  ph.de_switch = R(0);
    const R dh_safety = (R)safety*(R)dh;
+   if constexpr ( std::is_same<R,float>::value )
+   {
+      if ( !cfg_mhd( c ) && from_output && npatch >= 8*DT_PG_MIN && ( (uintptr_t)flu & 15u ) == 0 )
+      {
+         dt_cfl_pg_kernel<P><<< npatch/8, DT_PG_BLOCK, 0, st >>>( (const float*)flu, (float*)dt, ncomp, ph, dh_safety );
+         return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
+      }
+   }
    if ( cfg_mhd( c ) )
       dt_cfl_kernel<R,P,true><<< npatch, DT_BLOCK, 0, st >>>( (const R*)flu, (const R*)mag, (R*)dt, npatch,
                                                               from_output, ncomp, ph, dh_safety );
-   else if ( from_output && npatch >= 8*DT_PG_MIN && ( (uintptr_t)flu & 15u ) == 0 )
-      dt_cfl_pg_kernel<R,P><<< npatch/8, DT_PG_BLOCK, 0, st >>>( (const R*)flu, (R*)dt, ncomp, ph, dh_safety );
    else
       dt_cfl_kernel<R,P,false><<< npatch, DT_BLOCK, 0, st >>>( (const R*)flu, nullptr, (R*)dt, npatch,
                                                                from_output, ncomp, ph, dh_safety );
