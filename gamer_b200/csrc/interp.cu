@@ -188,36 +188,31 @@ struct IntArgs {
    int     *status;           // GB_INTERP_FAILED is OR-ed in where a parent still fails
 };
 
-// value of variable v of coarse cell q, conserved or (prim) primitive as Hydro_Con2Pri computes it
-// for Interpolate_Iterate (src/Interpolation/Interpolate.cpp:250-262; CPU_Shared_FluUtility.cpp:209-296)
+// the conserved variables u of a coarse cell in place of its primitive ones, as Hydro_Con2Pri computes
+// them for Interpolate_Iterate (src/Interpolation/Interpolate.cpp:250-262; CPU_Shared_FluUtility.cpp:209-296)
 template <typename R>
-GB_DEV R coarse_value( const IntArgs<R> &a, const R *cb, size_t c3, int v, int q, bool prim )
+GB_DEV void cell_primitive( const IntArgs<R> &a, R (&u)[5] )
 {
-   if ( !prim || v == 0 ) return cb[(size_t)v*c3 + q];
-   const R d = cb[q];
+   const R d = u[0], mx = u[1], my = u[2], mz = u[3];
    const R ird = rdiv( R(1), d );
-   if ( v < 4 ) return rmul( cb[(size_t)v*c3 + q], ird );
-   const R mx = cb[c3 + q], my = cb[2*c3 + q], mz = cb[3*c3 + q], e = cb[4*c3 + q];
+   u[1] = rmul( mx, ird );  u[2] = rmul( my, ird );  u[3] = rmul( mz, ird );
    // Hydro_Con2Eint, EoS_DensEint2Pres_Gamma, Hydro_CheckMinPres
-   const R eint = rsub( e, rdiv( rmul( R(0.5), radd( radd( rmul( mx, mx ), rmul( my, my ) ), rmul( mz, mz ) ) ), d ) );
+   const R eint = rsub( u[4], rdiv( rmul( R(0.5), radd( radd( rmul( mx, mx ), rmul( my, my ) ), rmul( mz, mz ) ) ), d ) );
    const R p = rmul( eint, a.gm1 );
-   return ( p == p ) ? rmax( p, a.min_pres ) : p;
+   u[4] = ( p == p ) ? rmax( p, a.min_pres ) : p;
 }
 
-// the eight children f[fz][fy][fx] of coarse cell (i, j, k) of batch item cb, variable v
+// the eight children f[fz][fy][fx] of the coarse cell c[0] of variable v; cx, cxy: strides along y and z
 template <int SCH, typename R>
-GB_DEV void children( const IntArgs<R> &a, const R *cb, size_t c3, int v, int i, int j, int k, bool prim, R coeff,
-                      R (&f)[2][2][2] )
+GB_DEV void children( const IntArgs<R> &a, const R *c, int cx, int cxy, int v, R coeff, R (&f)[2][2][2] )
 {
-   const int cx = a.csize[0], cxy = a.csize[0]*a.csize[1];
    const bool mono = ( a.mono >> v ) & 1u, opp = a.opp != 0;
    if constexpr ( SCH == INT_MINMOD1D )
    {
-      const int q = k*cxy + j*cx + i;
-      const R C = coarse_value( a, cb, c3, v, q, prim );
-      const R sx = minmod_slope( coarse_value( a, cb, c3, v, q - 1,   prim ), C, coarse_value( a, cb, c3, v, q + 1,   prim ), opp );
-      const R sy = minmod_slope( coarse_value( a, cb, c3, v, q - cx,  prim ), C, coarse_value( a, cb, c3, v, q + cx,  prim ), opp );
-      const R sz = minmod_slope( coarse_value( a, cb, c3, v, q - cxy, prim ), C, coarse_value( a, cb, c3, v, q + cxy, prim ), opp );
+      const R C = c[0];
+      const R sx = minmod_slope( c[-1],   C, c[1],   opp );
+      const R sy = minmod_slope( c[-cx],  C, c[cx],  opp );
+      const R sz = minmod_slope( c[-cxy], C, c[cxy], opp );
 #     pragma unroll
       for (int fz=0; fz<2; fz++)
 #     pragma unroll
@@ -240,9 +235,9 @@ GB_DEV void children( const IntArgs<R> &a, const R *cb, size_t c3, int v, int i,
       for (int yy=0; yy<W; yy++)
       {
          R line[W];
-         const int q = ( k + zz - G )*cxy + ( j + yy - G )*cx + i;
+         const R *q = c + ( zz - G )*cxy + ( yy - G )*cx;
 #        pragma unroll
-         for (int xx=0; xx<W; xx++) line[xx] = coarse_value( a, cb, c3, v, q + xx - G, prim );
+         for (int xx=0; xx<W; xx++) line[xx] = q[xx - G];
          op1d<SCH>( line, mono, coeff, opp, tx[zz][yy][0], tx[zz][yy][1] );
       }
       R ty[W][2][2];         // y pass: [z][fine y][fine x]
@@ -282,9 +277,10 @@ __global__ void interp_kernel( const __grid_constant__ IntArgs<R> a )
       const long long bv = t / ncell;
       const int v = (int)( bv % a.ncomp ), b = (int)( bv / a.ncomp );
       const int ii = c % nx, jj = ( c / nx ) % a.crange[1], kk = c / nxy;
-      const R *cb = a.cdata + (size_t)b*a.ncomp*c3;
+      const int cx = a.csize[0], cxy = a.csize[0]*a.csize[1];
+      const R *cb = a.cdata + ( (size_t)b*a.ncomp + v )*c3 + (size_t)( a.cstart[2] + kk )*cxy + ( a.cstart[1] + jj )*cx + a.cstart[0] + ii;
       R f[2][2][2];
-      children<SCH>( a, cb, c3, v, a.cstart[0] + ii, a.cstart[1] + jj, a.cstart[2] + kk, false, a.mono_coeff, f );
+      children<SCH>( a, cb, cx, cxy, v, a.mono_coeff, f );
       R *fb = a.fdata + ( (size_t)b*a.ncomp + v )*f3;
 #     pragma unroll
       for (int fz=0; fz<2; fz++)
@@ -325,162 +321,246 @@ GB_DEV bool child_fails( const IntArgs<R> &a, const R (&u)[5], bool prim )
    return bad;
 }
 
-// the attempts after the first of Interpolate_Iterate for one parent (primitive variables, then the
-// reduced coefficients), and the store of what they end with; the rare path, out of line so that the
-// first attempt keeps its children in registers.  (i, j, k): the parent in the coarse cells cb
-template <int SCH, typename R>
-__device__ __noinline__ void iterate_parent( const IntArgs<R> &a, const R *cb, size_t c3, int i, int j, int k, R *fo )
-{
-   const size_t fx = a.fsize[0], fxy = (size_t)a.fsize[0]*a.fsize[1], f3 = fxy*a.fsize[2];
-   const int mono_iter = a.mono_max_iter;
-   const int max_iter = a.int_prim ? mono_iter + 1 : mono_iter;
-   R f[5][2][2][2];
-   bool prim = false, ok = false;
-   R coeff = a.mono_coeff;
-   for (int it = 1; it <= max_iter && !ok; it++)
-   {
-      if ( it == 1 && a.int_prim ) prim = true;
-      else coeff = rmax( rsub( coeff, rdiv( a.mono_coeff, (R)mono_iter ) ), R(0) );
-#     pragma unroll 1
-      for (int v=0; v<5; v++) children<SCH>( a, cb, c3, v, i, j, k, prim, coeff, f[v] );
-      ok = true;
-#     pragma unroll 1
-      for (int q=0; q<8; q++)
-      {
-         R u[5];
-#        pragma unroll
-         for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
-         ok &= !child_fails( a, u, prim );
-      }
-   }
-   if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
-#  pragma unroll 1
-   for (int q=0; q<8; q++)
-   {
-      const int dz = q >> 2, dy = ( q >> 1 ) & 1, dx = q & 1;
-      R u[5];
-#     pragma unroll
-      for (int v=0; v<5; v++) u[v] = f[v][dz][dy][dx];
-      if ( prim )
-      {
-         // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
-         const R d = u[0];
-         u[1] = rmul( d, u[1] );  u[2] = rmul( d, u[2] );  u[3] = rmul( d, u[3] );
-         const R eint = rmul( u[4], a.inv_gm1 );
-         u[4] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( u[1], u[1] ), rmul( u[2], u[2] ) ), rmul( u[3], u[3] ) ) ), d ), eint );
-      }
-#     pragma unroll
-      for (int v=0; v<5; v++) fo[v*f3 + dz*fxy + dy*fx + dx] = u[v];
-   }
-}
-
 // Interpolate_Iterate for the five conserved hydro variables (INTERP_MASK: each parent on its own).
-// One CTA takes `depth` planes of parents of one region, so that the 27 (125) coarse cells around
-// each parent come from shared memory (STAGED; a region whose planes are too wide for that is read
-// from global memory).  The children of the five variables stay in registers: with a run-time loop
+// One CTA takes a box of parents of one region, or several whole regions where they are small, with
+// their coarse neighbourhoods in shared memory.  All parents of the CTA make the first attempt; those
+// with an unphysical child are listed and make the next one together, in full warps, until none is
+// left.  Before the second attempt the staged cells are turned into primitive variables in place, so
+// that no stencil has to.  The children of the five variables stay in registers: with a run-time loop
 // over the variables they went through local memory.  Bound by the issue of the 19 one-dimensional
-// operators of a parent's variable, each of rounded multiplications and selects.  With the assembly
-// below, 342 windows of 20^3, FP32: 217 -> 85 us (the bytes of both alone: 27 us).
+// operators of a parent's variable, each of rounded multiplications and selects.
+// cquad, FP32, us, against one thread per parent of the whole call that makes all its attempts from
+// global memory: 342 regions of 12^3 cells 97 -> 62, with half of the parents iterating 233 -> 131; 4096:
+// 1196 -> 695 and 2810 -> 1250; 8000 regions of 4^3 cells 25.4 -> 18.1 (with a CTA per region 252); one
+// of 70^3 87.5 -> 88.7; a call of a few thousand parents, which is latency, 10.1 -> 10.9.
 constexpr int INT_THREADS = 256;
 
 // CTAs per SM: 342 regions of 12^3 cells, with the window assembly, us: FP32 1: 137, 2: 111, 3: 97, 4: 103
 // (6 of 128 threads: 103); FP64 (229 regions) 1: 149, 2: 118, 3: 120, 4: 123
 template <typename R> constexpr int int_ctas() { return sizeof(R) == 4 ? 3 : 2; }
 
-template <int SCH, typename R, bool STAGED>
-__global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_kernel( const __grid_constant__ IntArgs<R> a, int depth, int nslab )
+// what a CTA takes: m whole regions, or (m = 1) one of nx x ny x nz boxes of n[] parents of a region
+struct IntTile {
+   int m, n[3], nbox[3];
+   int b[3], cells;            // coarse cells staged per variable, along each axis and in all
+   int list;                   // byte offset of the two lists of parents in shared memory
+   int threads;
+};
+
+template <int SCH, typename R>
+__global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_kernel( const __grid_constant__ IntArgs<R> a,
+                                                                                        const __grid_constant__ IntTile w )
 {
    constexpr int G = int_ghost( SCH );
    extern __shared__ __align__(16) unsigned char int_smem[];
-   const int b = blockIdx.x / nslab, k0 = ( blockIdx.x % nslab )*depth;
-   const int nk = ( a.crange[2] - k0 < depth ) ? a.crange[2] - k0 : depth;
-   const int nx = a.crange[0], nxy = a.crange[0]*a.crange[1], cxy = a.csize[0]*a.csize[1];
-   const size_t fx = a.fsize[0], fxy = (size_t)a.fsize[0]*a.fsize[1], f3 = fxy*a.fsize[2];
+   __shared__ int s_nfail[2];
+   R *s_c = (R*)int_smem;
+   const int tid = threadIdx.x, nth = blockDim.x;
+   const int nbox = w.nbox[0]*w.nbox[1]*w.nbox[2], box = blockIdx.x % nbox;
+   const int b0 = ( blockIdx.x / nbox )*w.m, nreg = ( a.nbatch - b0 < w.m ) ? a.nbatch - b0 : w.m;
+   // the box's first parent, its parents and its staged cells along each axis
+   const int o[3] = { ( box % w.nbox[0] )*w.n[0], ( box / w.nbox[0] % w.nbox[1] )*w.n[1], ( box / ( w.nbox[0]*w.nbox[1] ) )*w.n[2] };
+   int p[3];
+#  pragma unroll
+   for (int d=0; d<3; d++) p[d] = ( a.crange[d] - o[d] < w.n[d] ) ? a.crange[d] - o[d] : w.n[d];
+   const int sx = w.b[0], sxy = w.b[0]*w.b[1];
+   const int cx = a.csize[0], cxy = a.csize[0]*a.csize[1];
    const size_t c3 = (size_t)cxy*a.csize[2];
-   const R *cb = a.cdata + (size_t)b*5*c3;
-   const int n = ( nk + 2*G )*cxy;                                   // coarse cells staged per variable
-   const int kbase = STAGED ? a.cstart[2] + k0 - G : 0;              // their first plane
-   const size_t cs = STAGED ? (size_t)n : c3;
-   const R *src = STAGED ? (const R*)int_smem : cb;
-   if constexpr ( STAGED )
+   const int gx = a.cstart[0] + o[0] - G, gy = a.cstart[1] + o[1] - G, gz = a.cstart[2] + o[2] - G;
+   if ( tid < 2 ) s_nfail[tid] = 0;
+   if ( sx == cx && w.b[1] == a.csize[1] )
    {
-      R *s_c = (R*)int_smem;
-      const R *g = cb + (size_t)kbase*cxy;
-      // 16-byte loads where the array and whole planes are 16-byte aligned
+      // whole planes: one run per variable, or one in all for whole regions; 16-byte loads where every run
+      // starts on a 16-byte boundary
       constexpr int V = 16/sizeof(R);
-      if ( cxy % V == 0 && ( (uintptr_t)a.cdata & 15u ) == 0 )
+      const bool whole = ( w.b[2] == a.csize[2] );
+      const int nrun = whole ? 1 : 5*nreg, len = whole ? nreg*5*w.cells : ( p[2] + 2*G )*cxy;
+      const size_t first = (size_t)b0*5*c3 + (size_t)gz*cxy;
+      const bool vec = ( (uintptr_t)( a.cdata + first ) & 15u ) == 0 && ( nrun == 1 || ( c3 % V == 0 && w.cells % V == 0 ) );
+      for (int r=0; r<nrun; r++)
       {
-         for (int e = threadIdx.x; e < n/V; e += INT_THREADS)
-#           pragma unroll
-            for (int v=0; v<5; v++) ( (uint4*)( s_c + v*n ) )[e] = ( (const uint4*)( g + v*c3 ) )[e];
+         const R *src = a.cdata + first + r*c3;
+         R *dst = s_c + r*w.cells;
+         const int nv = vec ? len/V : 0;
+#        pragma unroll 4
+         for (int e = tid; e < nv; e += nth) ( (uint4*)dst )[e] = ( (const uint4*)src )[e];
+#        pragma unroll 4
+         for (int e = nv*V + tid; e < len; e += nth) dst[e] = src[e];
       }
-      else
-         for (int e = threadIdx.x; e < n; e += INT_THREADS)
-#           pragma unroll
-            for (int v=0; v<5; v++) s_c[v*n + e] = g[v*c3 + e];
-      __syncthreads();
    }
-   for (int c = threadIdx.x; c < nxy*nk; c += INT_THREADS)
+   else
    {
-      const int ii = c % nx, jj = ( c / nx ) % a.crange[1], kk = k0 + c / nxy;
-      const int i = a.cstart[0] + ii, j = a.cstart[1] + jj, k = a.cstart[2] + kk - kbase;
-      // Interpolate_Iterate stores from the origin of the fine region
-      R *fo = a.fdata + (size_t)b*5*f3 + (size_t)( 2*kk )*fxy + (size_t)( 2*jj )*fx + 2*ii;
-      R f[5][2][2][2];
-#     pragma unroll
-      for (int v=0; v<5; v++)
+      const int bx = p[0] + 2*G, bxy = bx*( p[1] + 2*G ), bn = bxy*( p[2] + 2*G );
+      for (int e = tid; e < nreg*bn; e += nth)
       {
-         children<SCH>( a, src, cs, v, i, j, k, false, a.mono_coeff, f[v] );
-         asm volatile( "" ::: "memory" );      // one variable's stencil live at a time
+         const int r = e / bn, c = e - r*bn, z = c / bxy, y = ( c - z*bxy ) / bx, x = c - z*bxy - y*bx;
+         const R *src = a.cdata + (size_t)( b0 + r )*5*c3 + (size_t)( gz + z )*cxy + (size_t)( gy + y )*cx + gx + x;
+         R *dst = s_c + r*5*w.cells + z*sxy + y*sx + x;
+#        pragma unroll
+         for (int v=0; v<5; v++) dst[v*w.cells] = src[v*c3];
       }
-      bool ok = true;
-#     pragma unroll
-      for (int q=0; q<8; q++)
+   }
+   __syncthreads();
+
+   const size_t fx = a.fsize[0], fxy = (size_t)a.fsize[0]*a.fsize[1], f3 = fxy*a.fsize[2];
+   const int np = p[0]*p[1]*p[2], mono_iter = a.mono_max_iter, max_iter = a.int_prim ? mono_iter + 1 : mono_iter;
+   unsigned short *list = (unsigned short*)( int_smem + w.list );        // [2][the CTA's parents]
+   const int nlist = w.m*w.n[0]*w.n[1]*w.n[2];
+   R coeff = a.mono_coeff;
+   bool prim = false;
+   int n = nreg*np;
+   for (int it=0; ; it++)
+   {
+      const unsigned short *cur = list + ( it & 1 )*nlist;
+      unsigned short *next = list + ( ( it + 1 ) & 1 )*nlist;
+      for (int e = tid; e < n; e += nth)
       {
-         R u[5];
+         const int id = ( it == 0 ) ? e : cur[e];
+         const int r = id / np, c = id - r*np;
+         const int ii = c % p[0], jj = c / p[0] % p[1], kk = c / ( p[0]*p[1] );
+         const R *src = s_c + r*5*w.cells + ( kk + G )*sxy + ( jj + G )*sx + ii + G;
+         R f[5][2][2][2];
 #        pragma unroll
-         for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
-         ok &= !child_fails( a, u, false );
+         for (int v=0; v<5; v++)
+         {
+            children<SCH>( a, src + v*w.cells, sx, sxy, v, coeff, f[v] );
+            asm volatile( "" ::: "memory" );      // one variable's stencil live at a time
+         }
+         bool ok = true;
+#        pragma unroll
+         for (int q=0; q<8; q++)
+         {
+            R u[5];
+#           pragma unroll
+            for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+            ok &= !child_fails( a, u, prim );
+         }
+         if ( !ok && it < max_iter ) { next[atomicAdd( &s_nfail[it & 1], 1 )] = (unsigned short)id;  continue; }
+         if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
+         // Interpolate_Iterate stores from the origin of the fine region
+         R *fo = a.fdata + (size_t)( b0 + r )*5*f3 + (size_t)( 2*( o[2] + kk ) )*fxy + (size_t)( 2*( o[1] + jj ) )*fx + 2*( o[0] + ii );
+#        pragma unroll
+         for (int q=0; q<8; q++)
+         {
+            R u[5];
+#           pragma unroll
+            for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+            if ( prim )
+            {
+               // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
+               const R d = u[0];
+               u[1] = rmul( d, u[1] );  u[2] = rmul( d, u[2] );  u[3] = rmul( d, u[3] );
+               const R eint = rmul( u[4], a.inv_gm1 );
+               u[4] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( u[1], u[1] ), rmul( u[2], u[2] ) ), rmul( u[3], u[3] ) ) ), d ), eint );
+            }
+#           pragma unroll
+            for (int v=0; v<5; v++) fo[v*f3 + ( q >> 2 )*fxy + ( ( q >> 1 ) & 1 )*fx + ( q & 1 )] = u[v];
+         }
       }
-      if ( !ok ) { iterate_parent<SCH>( a, src, cs, i, j, k, fo );  continue; }
-#     pragma unroll
-      for (int v=0; v<5; v++)
-#        pragma unroll
-         for (int q=0; q<8; q++) fo[v*f3 + ( q >> 2 )*fxy + ( ( q >> 1 ) & 1 )*fx + ( q & 1 )] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+      if ( it == max_iter ) return;
+      __syncthreads();
+      n = s_nfail[it & 1];
+      if ( n == 0 ) return;
+      if ( tid == 0 ) s_nfail[( it + 1 ) & 1] = 0;
+      if ( it == 0 && a.int_prim )
+      {
+         for (int e = tid; e < nreg*w.cells; e += nth)
+         {
+            R *q = s_c + ( e / w.cells )*5*w.cells + e % w.cells, u[5];
+#           pragma unroll
+            for (int v=0; v<5; v++) u[v] = q[v*w.cells];
+            cell_primitive( a, u );
+#           pragma unroll
+            for (int v=0; v<5; v++) q[v*w.cells] = u[v];
+         }
+         prim = true;
+      }
+      else coeff = rmax( rsub( coeff, rdiv( a.mono_coeff, (R)mono_iter ) ), R(0) );
+      __syncthreads();
    }
 }
 
-// planes of parents per CTA and their shared memory: half the parents' planes, fewer where those need
-// more than 48 KB (four CTAs share an SM) or where few regions would leave SMs idle, one at least;
-// 0 bytes where even that needs over 200 KB
+// The boxes of a call.  A round of 256 parents on an SM that holds a full set of CTAs takes one unit of
+// time, alone on its SM `alone` units (measured for 12^3 regions: 8.3 and 11.7 us in FP32, 15 us both
+// in FP64), the staging of 256 cells 0.06 (of a cell by one thread 0.03) and the launch of a CTA 0.05; the choice is the one for which the slowest SM, or the
+// chain of rounds of the CTAs that follow each other in one place, takes least, and the largest box
+// of those that tie.  At most 48 KB of shared memory.
 template <typename R>
-int interp_depth( int scheme, const IntArgs<R> &a, size_t *smem )
+IntTile interp_tile( int scheme, const IntArgs<R> &a, int nsm )
 {
    const int G = int_ghost( scheme );
-   const size_t plane = (size_t)5*a.csize[0]*a.csize[1]*sizeof(R);
-   int depth = ( a.crange[2] + 1 )/2;
-   while ( depth > 1 && (long long)a.nbatch*( ( a.crange[2] + depth - 1 )/depth ) < 296 ) depth = ( depth + 1 )/2;
-   while ( depth > 1 && ( depth + 2*G )*plane > 48*1024 ) depth--;
-   *smem = ( depth + 2*G )*plane;
-   if ( *smem > 200*1024 ) *smem = 0;
-   return depth;
+   const double alone = ( sizeof(R) == 4 ) ? 1.4 : 1.0;
+   constexpr int SMEM = 48*1024 - 64;
+   const int nx = a.crange[0], ny = a.crange[1], nz = a.crange[2];
+   const long long region = (long long)nx*ny*nz;
+   IntTile best;
+   best.m = 0;
+   double best_cost = 0.0;
+   // m regions, or a box of px x py x pz parents; whether it fits
+   auto consider = [&]( int m, int px, int py, int pz )
+   {
+      const long long cells = (long long)( px + 2*G )*( py + 2*G )*( pz + 2*G ), parents = (long long)m*px*py*pz;
+      const long long list = ( 5*m*cells*(long long)sizeof(R) + 15 )/16*16;
+      if ( list + 4*parents > SMEM || parents > 65535 ) return false;
+      IntTile t;
+      t.m = m;
+      t.n[0] = px;  t.n[1] = py;  t.n[2] = pz;
+      for (int d=0; d<3; d++) { t.nbox[d] = ( a.crange[d] + t.n[d] - 1 )/t.n[d];  t.b[d] = t.n[d] + 2*G; }
+      t.cells = (int)cells;
+      t.list  = (int)list;
+      const int warps = ( parents >= INT_THREADS ) ? INT_THREADS/32 : (int)( parents + 31 )/32;
+      t.threads = 32*warps;
+      const int rounds = (int)( ( parents + t.threads - 1 )/t.threads );
+      // CTAs that share an SM: by registers and by shared memory
+      int share = int_ctas<R>()*( INT_THREADS/32 )/warps;
+      const int fit = 227*1024/( t.list + 4*(int)parents + 1024 );
+      if ( fit < share ) share = fit;
+      const long long ctas = (long long)t.nbox[0]*t.nbox[1]*t.nbox[2]*( ( a.nbatch + m - 1 )/m );
+      const long long per_sm = ( ctas + nsm - 1 )/nsm, waves = ( per_sm + share - 1 )/share;
+      // threads beyond the parents stage the cells with fewer loads one after the other, where an SM has few CTAs
+      int more = ( per_sm <= int_ctas<R>() ) ? INT_THREADS/32 : 0;
+      if ( more > ( m*cells + 31 )/32 ) more = (int)( ( m*cells + 31 )/32 );
+      if ( more > warps ) t.threads = 32*more;
+      const double load = per_sm*( warps*rounds/8.0 + 0.06*m*cells/256 );
+      const double chain = waves*( alone*rounds + 0.03*m*cells/t.threads );
+      const double cost = ( ( load > chain ) ? load : chain ) + 0.05*per_sm;
+      if ( best.m == 0 || cost < best_cost ) { best = t;  best_cost = cost; }
+      return true;
+   };
+   // small regions: several, at most two rounds
+   if ( region <= INT_THREADS )
+      for (int m = ( a.nbatch < 2*INT_THREADS/(int)region ) ? a.nbatch : 2*INT_THREADS/(int)region; m > 1; m -= 1 + m/8) consider( m, nx, ny, nz );
+   // whole planes, or boxes cut along y too where the planes are too large or too few for the SMs; along x
+   // where not even one row fits, or only a box with less than a round of parents for a large region
+   bool fits = false;
+   for (int kx = 1; ; kx *= 2)
+   {
+      const int px = ( nx + kx - 1 )/kx;
+      for (int ky = 1; ; ky *= 2)
+      {
+         const int py = ( ny + ky - 1 )/ky;
+         int last = 0;
+         for (int kz = 1; kz < 16 && kz <= nz; kz++)
+         {
+            const int pz = ( nz + kz - 1 )/kz;
+            if ( pz != last ) fits |= consider( 1, px, py, pz );
+            last = pz;
+         }
+         if ( last != 1 ) fits |= consider( 1, px, py, 1 );
+         if ( py == 1 || ( fits && (long long)a.nbatch*ky*nz >= 2*nsm ) ) break;
+      }
+      if ( px == 1 || ( fits && ( px < 32 || best.threads == INT_THREADS || region*a.nbatch < (long long)nsm*INT_THREADS ) ) ) return best;
+   }
 }
 
 template <int SCH, typename R>
-cudaError_t iterate_launch( const IntArgs<R> &a, cudaStream_t st )
+cudaError_t iterate_launch( const IntArgs<R> &a, int nsm, cudaStream_t st )
 {
-   size_t smem = 0;
-   const int depth = interp_depth( SCH, a, &smem ), nslab = ( a.crange[2] + depth - 1 )/depth;
-   const long long grid = (long long)nslab*a.nbatch;
+   const IntTile t = interp_tile( SCH, a, nsm );
+   const long long grid = (long long)t.nbox[0]*t.nbox[1]*t.nbox[2]*( ( a.nbatch + t.m - 1 )/t.m );
    if ( grid > 0x7fffffffLL ) return cudaErrorInvalidValue;
-   if ( smem == 0 ) interp_iterate_kernel<SCH,R,false><<< (unsigned)grid, INT_THREADS, 0, st >>>( a, depth, nslab );
-   else
-   {
-      const cudaError_t e = ( smem <= 48*1024 ) ? cudaSuccess
-         : cudaFuncSetAttribute( interp_iterate_kernel<SCH,R,true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200*1024 );
-      if ( e != cudaSuccess ) return e;
-      interp_iterate_kernel<SCH,R,true><<< (unsigned)grid, INT_THREADS, smem, st >>>( a, depth, nslab );
-   }
+   const size_t smem = t.list + (size_t)4*t.m*t.n[0]*t.n[1]*t.n[2];
+   interp_iterate_kernel<SCH,R><<< (unsigned)grid, t.threads, smem, st >>>( a, t );
    return cudaGetLastError();
 }
 
@@ -497,7 +577,7 @@ cudaError_t interp_launch( int scheme, bool iterate, const IntArgs<R> &a, cudaSt
    if ( g > 32LL*nsm ) g = 32LL*nsm;
    if ( g < 1 ) return cudaSuccess;
 #  define GB_INT_CASE( S ) \
-   case S: if ( iterate ) return iterate_launch<S,R>( a, st ); \
+   case S: if ( iterate ) return iterate_launch<S,R>( a, nsm, st ); \
            interp_kernel<S,R><<< (unsigned)g, B, 0, st >>>( a );  break;
    switch ( scheme )
    {
