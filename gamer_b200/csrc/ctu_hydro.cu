@@ -347,11 +347,13 @@ size_t ctu_hydro_scratch_bytes_per_pg( int precision, int ncomp, int lr_scheme )
    return hctu_scratch_per_pg( ( precision == GB_PREC_FP64 ) ? 8 : 4, ncomp, lr_scheme );
 }
 
-// one hydro CTU solve of npg patch groups in chunks of scratch_bytes / ctu_hydro_scratch_bytes_per_pg
-int ctu_hydro_solve( const gb_fluid_config &cfg, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
+// one hydro CTU solve of npg patch groups: by the plane-streaming kernel (fused: ctu_hydro_fused of the
+// caller's whole call, of which these may be a chunk), or by the separate kernels in chunks of
+// scratch_bytes / ctu_hydro_scratch_bytes_per_pg
+int ctu_hydro_solve( const gb_fluid_config &cfg, bool fused, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
                      const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, int *status, cudaStream_t st )
 {
-   if ( ctu_hydro_fused( cfg, npg ) )
+   if ( fused )
    {
       if ( cfg.precision == GB_PREC_FP64 )  return ctu_fused_fp64 ( cfg, flu_in, flu_out, flux, npg, prm, status, st );
       if ( cfg.precision == GB_PREC_MIXED ) return ctu_fused_mixed( cfg, flu_in, flu_out, flux, npg, prm, status, st );

@@ -46,7 +46,7 @@ size_t mhm_mhd_scratch_bytes_per_pg( int precision );
 size_t ctu_ppm_mhd_scratch_bytes_per_pg( int precision );
 size_t mhm_ppm_mhd_scratch_bytes_per_pg( int precision );
 size_t ctu_hydro_scratch_bytes_per_pg( int precision, int ncomp, int lr_scheme );
-int ctu_hydro_solve( const gb_fluid_config &cfg, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
+int ctu_hydro_solve( const gb_fluid_config &cfg, bool fused, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
                      const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, int *status, cudaStream_t st );
 bool ctu_hydro_fused( const gb_fluid_config &cfg, int npg );
 int ctu_solve( const gb_fluid_config &cfg, const void *flu_in, const void *mag_in, void *flu_out, void *mag_out,
@@ -351,11 +351,15 @@ int solve_host_ctu( gb_fluid_solver *s, const void *flu_in, void *flu_out, const
    int chunk = ( mhd_chunk( s ) < GB_HOST_CTU_CHUNK ) ? mhd_chunk( s ) : GB_HOST_CTU_CHUNK;
    if ( npg < chunk ) chunk = npg;
    const bool dual = ( s->cfg.dual_energy == GB_DE_ENPY );
+   // the kernel is chosen by the patch groups of the whole call, so that every chunk rounds alike (and like
+   // the same call on device arrays); the plane-streaming one needs no scratch
+   const bool fused = !is_mhd( s ) && gb::ctu_hydro_fused( s->cfg, npg );
    const size_t bd = (size_t)PS2*PS2*PS2;
    int rc = ensure_staging( s, chunk );
    if ( rc != GB_OK ) return rc;
-   for (int q=0; q<gb_fluid_solver::NSTREAM; q++)
-      if ( ( rc = ensure_scratch( s, q, chunk ) ) != GB_OK ) return rc;
+   if ( !fused )
+      for (int q=0; q<gb_fluid_solver::NSTREAM; q++)
+         if ( ( rc = ensure_scratch( s, q, chunk ) ) != GB_OK ) return rc;
    const size_t scratch_chunk = ctu_per_pg( s )*(size_t)chunk;
    const size_t bi = in_bytes_pg( s ), bo = out_bytes_pg( s ), bf = flx_bytes_pg( s );
    const size_t bbi = bin_bytes_pg( s ), bbo = bout_bytes_pg( s ), be = ele_bytes_pg( s );
@@ -379,7 +383,7 @@ int solve_host_ctu( gb_fluid_solver *s, const void *flu_in, void *flu_out, const
          if ( dual && de_out &&
               cudaMemcpyAsync( s->d_de[q], de_out + p0*bd, n*bd, cudaMemcpyHostToDevice, st ) != cudaSuccess )
             return GB_E_CUDA;
-         rc = gb::ctu_hydro_solve( s->cfg, s->d_in[q], s->d_out[q], prm->store_flux ? s->d_flux[q] : nullptr,
+         rc = gb::ctu_hydro_solve( s->cfg, fused, s->d_in[q], s->d_out[q], prm->store_flux ? s->d_flux[q] : nullptr,
                                    ( dual && de_out ) ? s->d_de[q] : nullptr, n, prm, s->d_scratch[q], scratch_chunk,
                                    s->d_status, st );
       }
@@ -792,10 +796,11 @@ int gb_fluid_solve_device( gb_fluid_solver *s, const void *flu_in, void *flu_out
    if ( is_ctu( s ) )
    {
       // the plane-streaming kernel needs no scratch
-      const int chunk = gb::ctu_hydro_fused( s->cfg, npg ) ? 0 : ( npg < mhd_chunk( s ) ) ? npg : mhd_chunk( s );
+      const bool fused = gb::ctu_hydro_fused( s->cfg, npg );
+      const int chunk = fused ? 0 : ( npg < mhd_chunk( s ) ) ? npg : mhd_chunk( s );
       if ( chunk > 0 && ( rc = ensure_scratch( s, 0, chunk ) ) != GB_OK ) return rc;
       s->last = (cudaStream_t)stream;
-      return gb::ctu_hydro_solve( s->cfg, flu_in, flu_out, prm->store_flux ? flux : nullptr, de_out, npg, prm,
+      return gb::ctu_hydro_solve( s->cfg, fused, flu_in, flu_out, prm->store_flux ? flux : nullptr, de_out, npg, prm,
                                   s->d_scratch[0], ctu_per_pg( s )*(size_t)chunk, s->d_status, (cudaStream_t)stream );
    }
    if ( is_rp( s ) )

@@ -130,7 +130,12 @@ int gb_fluid_destroy( gb_fluid_solver *s );
  * (src/Model_Hydro/CPU_Hydro/CPU_FluidSolver_CTU.cpp:157-342): hydro (PLM, characteristic tracing,
  * HLLC or HLLE) or MHD (PLM, HLLD with the HLLE rescue, constrained transport; needs mag_in and
  * mag_out).
- * pg_fail (optional, int[npg]) receives 1 for each patch group still unphysical after the retries. */
+ * pg_fail (optional, int[npg]) receives 1 for each patch group still unphysical after the retries.
+ * A patch group's result does not depend on the others of the call, with one exception: hydro CTU
+ * (five variables, primitive limiting) runs as one kernel when the call has enough patch groups and as
+ * several kernels otherwise, and the two may differ in the last bits.  npg and the configuration
+ * decide, so that the host-array calls below give the bits of this call whatever their chunks; a batch
+ * split over calls of other sizes need not. */
 int gb_fluid_solve_device( gb_fluid_solver *s, const void *flu_in, void *flu_out,
                            const void *mag_in, void *mag_out, char *de_out,
                            void *flux, void *ele, int *pg_fail, int npg,
@@ -212,7 +217,9 @@ int gb_fluid_get_launch( gb_fluid_solver *s, int *threads, int *ctas_per_sm, int
  * mixed, 1024 in FP64; the host-array entry point uses at most 512, to pipeline its copies).
  * Each stream slot holds a device scratch of ~2.8 MB (MHD, FP32; hydro ~1.2 MB; twice that in
  * FP64) per patch group of the largest chunk used so far (a call of fewer patch groups than the
- * chunk needs only those), allocated on first use.  Concurrent calls on one solver share the
+ * chunk needs only those), allocated on first use.  The hydro calls that run as one kernel (see
+ * gb_fluid_solve_device) use no scratch: on device arrays they are not chunked, on host arrays the chunk
+ * is that of the copies.  Concurrent calls on one solver share the
  * scratch of the device entry point and must not overlap. */
 int gb_fluid_set_mhd_chunk( gb_fluid_solver *s, int npg );
 
@@ -355,7 +362,10 @@ int gb_fluid_get_config( const gb_fluid_solver *s, gb_fluid_config *cfg );
  * d loss / d flu_in for the same flu_in.  Supported: MHM + PLM, GMinMod with MinMod_Coeff < 2, no
  * retries, no dual energy, FLU_NXT = 20, GB_PREC_FP32 (double accumulation) or GB_PREC_FP64.
  * The caller provides the device workspace (gb_fluid_adjoint_workspace_bytes per batch; a smaller
- * workspace is used in chunks of patch groups, at least one patch group's worth is required). */
+ * workspace is used in chunks of patch groups, at least one patch group's worth is required).
+ * FP32 with HLLC runs as one kernel where npg fills two thirds of the waves of one patch group per SM
+ * (and the arrays are 16-byte aligned), as several kernels otherwise; the two agree to rounding (the
+ * face states may differ in their last bit), not bit for bit. */
 int gb_fluid_adjoint_workspace_bytes( const gb_fluid_solver *s, int npg, unsigned long long *bytes );
 int gb_fluid_adjoint_step_device( gb_fluid_solver *s, const void *flu_in, const double *gout, double *gin, int npg,
                                   const gb_fluid_params *prm, void *workspace, unsigned long long ws_bytes,

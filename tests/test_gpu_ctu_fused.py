@@ -70,3 +70,21 @@ def test_streaming_kernel_without_flux_planes(cuda_device):
     a, _ = _solve(s, x, SolverParams(dt=dt, dh=dh), 125)
     b, f = _solve(s, x, SolverParams(dt=dt, dh=dh, StoreFlux=False), 125)
     assert torch.equal(a, b) and bool(torch.isnan(f).all())
+
+
+@pytest.mark.parametrize("prec,npg,chunk", [("fp32", 560, 0), ("fp32", 560, 100), ("fp32", 60, 7), ("mixed", 600, 0), ("fp64", 520, 0)])
+def test_host_calls_equal_device_calls_whatever_the_chunks(cuda_device, prec, npg, chunk):
+    """The kernel is chosen once for a call: neither the chunks of the host-array entry point (512, or
+    fewer) nor a last, small chunk give other bits than the same call on device arrays."""
+    import torch
+    box = ic.lognormal_box(4, seed=npg, gamma=GAMMA)
+    dh = 1.0 / 64
+    s = FluidSolver(scheme="ctu", precision=prec, gamma=GAMMA)
+    x = ic.cut_patch_groups(box, 20).astype(s.np_dtype)
+    x = np.concatenate([x] * (-(-npg // x.shape[0])))[:npg]
+    prm = SolverParams(dt=ic.cfl_dt(box, GAMMA, dh, cfl=0.4), dh=dh)
+    out, flux = _solve(s, torch.from_numpy(x).cuda(), prm, npg)
+    if chunk:
+        s.set_mhd_chunk(chunk)
+    hout, hflux, _ = s.solve_host(x, prm)
+    assert np.array_equal(hout, out.cpu().numpy()) and np.array_equal(hflux, flux.cpu().numpy())
