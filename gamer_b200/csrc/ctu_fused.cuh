@@ -473,33 +473,35 @@ cudaError_t hctu_fused_launch( const hctu::Args<R> &a, int *status, cudaStream_t
    return cudaGetLastError();
 }
 
-// a call of one precision policy: the solver, reconstruction and limiter kinds it is built for
+// a call of one precision policy: the solvers, reconstructions and limiter kinds that ctu_hydro_fused has a
+// line for
 template <typename R, int P, int RS, int LR>
 int hctu_fused_call( const gb_fluid_config &cfg, const void *in, void *out, void *flux, int npg, const gb_fluid_params *prm,
                      int *status, cudaStream_t st )
 {
    const hctu::Args<R> a = hctu_args<R,5,LR>( cfg, in, out, flux, nullptr, 0, npg, prm );
-   const bool gmm = ( prm->lr_limiter == GB_LIM_GMINMOD && prm->minmod_coeff < 2.0 );
-   const cudaError_t e = gmm ? hctu_fused_launch<R,P,RS,LR,true>( a, status, st )
-                             : hctu_fused_launch<R,P,RS,LR,false>( a, status, st );
-   return ( e == cudaSuccess ) ? GB_OK : GB_E_CUDA;
+   if ( hctu_gmm( *prm ) ) return ( hctu_fused_launch<R,P,RS,LR,true>( a, status, st ) == cudaSuccess ) ? GB_OK : GB_E_CUDA;
+   if constexpr ( P != P_MIXED && !( LR == LR_PPM && RS == RS_HLLE ) )
+      return ( hctu_fused_launch<R,P,RS,LR,false>( a, status, st ) == cudaSuccess ) ? GB_OK : GB_E_CUDA;
+   return GB_E_UNSUPPORTED;
 }
 
 template <typename R, int P>
 int hctu_fused_pick( const gb_fluid_config &cfg, const void *in, void *out, void *flux, int npg, const gb_fluid_params *prm,
                      int *status, cudaStream_t st )
 {
-   const bool ppm = ( cfg.lr_scheme == GB_LR_PPM );
-   constexpr int LRP = ( sizeof(R) == 4 ) ? LR_PPM : LR_PLM;     // PPM in FP64 needs 266 KB of shared memory: not built
-   if ( ppm && LRP != LR_PPM ) return GB_E_UNSUPPORTED;
-#  define GB_FUSED( RS ) \
-   return ppm ? hctu_fused_call<R,P,RS,LRP>( cfg, in, out, flux, npg, prm, status, st ) \
-              : hctu_fused_call<R,P,RS,LR_PLM>( cfg, in, out, flux, npg, prm, status, st )
-   if ( cfg.rsolver == GB_RSOLVER_HLLC ) GB_FUSED( RS_HLLC );
-   if ( cfg.rsolver == GB_RSOLVER_HLLE ) GB_FUSED( RS_HLLE );
-   if ( cfg.rsolver == GB_RSOLVER_ROE  ) GB_FUSED( RS_ROE );
-#  undef GB_FUSED
-   return GB_E_UNSUPPORTED;
+   if ( cfg.rsolver != GB_RSOLVER_HLLC && cfg.rsolver != GB_RSOLVER_HLLE ) return GB_E_UNSUPPORTED;
+   const bool hlle = ( cfg.rsolver == GB_RSOLVER_HLLE );
+   if ( cfg.lr_scheme == GB_LR_PPM )
+   {
+      if constexpr ( P == P_FP32 )
+         return hlle ? hctu_fused_call<R,P,RS_HLLE,LR_PPM>( cfg, in, out, flux, npg, prm, status, st )
+                     : hctu_fused_call<R,P,RS_HLLC,LR_PPM>( cfg, in, out, flux, npg, prm, status, st );
+      else
+         return GB_E_UNSUPPORTED;
+   }
+   return hlle ? hctu_fused_call<R,P,RS_HLLE,LR_PLM>( cfg, in, out, flux, npg, prm, status, st )
+               : hctu_fused_call<R,P,RS_HLLC,LR_PLM>( cfg, in, out, flux, npg, prm, status, st );
 }
 
 } // namespace gb

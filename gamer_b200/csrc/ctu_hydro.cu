@@ -233,25 +233,38 @@ __global__ void hctu_update( const __grid_constant__ hctu::Args<R> a )
    }
 }
 
-// Whether a call of npg patch groups runs through the plane-streaming kernel: five variables, limiting
-// in primitive variables, and HLLC, HLLE or Roe (PPM: not with Roe, 2.13 against 2.00 ms at 1000
-// patch groups; not in FP64, whose planes need 266 KB of shared memory).
-// It takes one time T per wave of patch groups (one or two CTAs per SM), 19 dependent steps long,
-// while the separate kernels spread any number over the whole GPU and take a time t per patch group:
-// the line lies at npg = T/t per wave.  Measured on B200, us: FP32 PLM HLLC T 121, t 1.21 (100 patch
-// groups: 121 / 129, 40: 121 / 59, 4096: 2030 / 4364); PPM T 176, t 1.77; FP64 T 211, t 2.08 (1000:
-// 1461 / 2079).  Mixed T 234, t 1.13 on a flow where every cell takes the double recovery; Roe T 285, t
-// 1.23 (1000: 1141 / 1232).
-bool ctu_hydro_fused( const gb_fluid_config &cfg, int npg )
+// Whether a call of npg patch groups runs through the plane-streaming kernel (ctu_fused.cuh): five
+// variables, limiting in primitive variables, HLLC or HLLE, and PLM, or PPM in FP32.
+// It takes one time T per wave of patch groups (two CTAs per SM for PLM in float, one otherwise), 19
+// dependent steps long, while the separate kernels spread any number over the whole GPU and take a time t
+// per patch group: the line lies at npg = T/t per wave, with T from the slowest of a lognormal, a
+// Kelvin-Helmholtz and a blast flow, for generalized MinMod with theta < 2 (built in) and for the other
+// limiters (chosen at run time).  Measured on B200, us, streaming / separate:
+//    FP32 PLM        MinMod 100 patch groups 122 / 127, 40: 123 / 60, 592: 312 / 653; others (van Albada)
+//                    125: 164 / 165, 290: 204 / 354, but 297 to 310 a few us more than the separate ones
+//    FP32 PPM HLLC   MinMod 100: 181 / 181, 592: 706 / 981; others 125: 261 / 248, 290: 515 / 551
+//    FP32 PPM HLLE   MinMod 100: 192 / 179, 120: 193 / 217, 592: 756 / 979; others no gain (1000: 1850 / 1795)
+//    mixed PLM       MinMod T 236 lognormal, 263 blast, t 1.08 (592: 474 / 664); others no gain (blast 580: 769 / 678)
+//    FP64 PLM        MinMod 100: 210 / 232, 592: 834 / 1190; others 290: 565 / 646, blast 1000: 2154 / 2113
+// Not built, since no line holds for every flow: Roe (its reference states lengthen the chain; lognormal
+// FP32 592: 847 / 797, mixed 1334 / 978, FP64 1848 / 1662; Kelvin-Helmholtz 616 / 740, 756 / 752, 1361 / 1481),
+// and PPM in mixed (one CTA per SM; 2000: 3381 / 3233, blast 1000: 1939 / 1638, Kelvin-Helmholtz 1068 / 1469).
+// PPM in FP64 would need 266 KB of shared memory.
+bool ctu_hydro_fused( const gb_fluid_config &cfg, const gb_fluid_params &prm, int npg )
 {
-   const bool ppm = ( cfg.lr_scheme == GB_LR_PPM ), fp64 = ( cfg.precision == GB_PREC_FP64 );
+   const bool ppm = ( cfg.lr_scheme == GB_LR_PPM ), hlle = ( cfg.rsolver == GB_RSOLVER_HLLE ), gmm = hctu_gmm( prm );
    if ( cfg.dual_energy != GB_DE_NONE || cfg.npassive_user != 0 || cfg.char_reconstruction ) return false;
-   if ( cfg.rsolver == GB_RSOLVER_EXACT || ( ppm && ( fp64 || cfg.rsolver == GB_RSOLVER_ROE ) ) ) return false;
+   if ( ( cfg.rsolver != GB_RSOLVER_HLLC && !hlle ) || ( ppm && cfg.precision != GB_PREC_FP32 ) ) return false;
+   int line;
+   if      ( cfg.precision == GB_PREC_MIXED ) { if ( !gmm ) return false;  line = 245; }
+   else if ( cfg.precision == GB_PREC_FP64 )  line = gmm ? 100 : 144;
+   else if ( ppm && hlle )                    { if ( !gmm ) return false;  line = 110; }
+   else if ( ppm )                            line = gmm ? 105 : 140;
+   else                                       line = gmm ? 100 : 155;
    int dev = 0, nsm = 148;
    cudaGetDevice( &dev );
    cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
-   const int slots = nsm*( ( ppm || fp64 ) ? 1 : 2 ), waves = ( npg + slots - 1 )/slots;
-   const int line = ( !fp64 && ( cfg.precision == GB_PREC_MIXED || cfg.rsolver != GB_RSOLVER_HLLC ) ) ? 235 : 100;
+   const int slots = nsm*( ( ppm || cfg.precision == GB_PREC_FP64 ) ? 1 : 2 ), waves = ( npg + slots - 1 )/slots;
    return npg > 0 && npg >= line*waves;
 }
 
@@ -367,3 +380,10 @@ int ctu_hydro_solve( const gb_fluid_config &cfg, bool fused, const void *flu_in,
 }
 
 } // namespace gb
+
+extern "C" int gb_fluid_ctu_one_kernel( const gb_fluid_config *cfg, const gb_fluid_params *prm, int npg, int *one )
+{
+   if ( cfg == nullptr || prm == nullptr || one == nullptr || npg < 0 ) return GB_E_INVALID;
+   *one = ( cfg->scheme == GB_SCHEME_CTU && cfg->rsolver != GB_RSOLVER_HLLD && gb::ctu_hydro_fused( *cfg, *prm, npg ) ) ? 1 : 0;
+   return GB_OK;
+}

@@ -8,6 +8,9 @@
 
 namespace gb {
 
+// generalized MinMod with theta < 2, which the plane-streaming kernel has built in
+inline bool hctu_gmm( const gb_fluid_params &prm ) { return prm.lr_limiter == GB_LIM_GMINMOD && (float)prm.minmod_coeff < 2.0f; }
+
 namespace hctu {
 constexpr int NX  = 20;                // FLU_NXT
 constexpr int NX3 = NX*NX*NX;

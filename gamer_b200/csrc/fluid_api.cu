@@ -48,7 +48,7 @@ size_t mhm_ppm_mhd_scratch_bytes_per_pg( int precision );
 size_t ctu_hydro_scratch_bytes_per_pg( int precision, int ncomp, int lr_scheme );
 int ctu_hydro_solve( const gb_fluid_config &cfg, bool fused, const void *flu_in, void *flu_out, void *flux, char *de, int npg,
                      const gb_fluid_params *prm, void *scratch, size_t scratch_bytes, int *status, cudaStream_t st );
-bool ctu_hydro_fused( const gb_fluid_config &cfg, int npg );
+bool ctu_hydro_fused( const gb_fluid_config &cfg, const gb_fluid_params &prm, int npg );
 int ctu_solve( const gb_fluid_config &cfg, const void *flu_in, const void *mag_in, void *flu_out, void *mag_out,
                void *flux, void *ele, int npg, const gb_fluid_params *prm, void *scratch, size_t scratch_bytes,
                cudaStream_t st );
@@ -353,7 +353,7 @@ int solve_host_ctu( gb_fluid_solver *s, const void *flu_in, void *flu_out, const
    const bool dual = ( s->cfg.dual_energy == GB_DE_ENPY );
    // the kernel is chosen by the patch groups of the whole call, so that every chunk rounds alike (and like
    // the same call on device arrays); the plane-streaming one needs no scratch
-   const bool fused = !is_mhd( s ) && gb::ctu_hydro_fused( s->cfg, npg );
+   const bool fused = !is_mhd( s ) && gb::ctu_hydro_fused( s->cfg, *prm, npg );
    const size_t bd = (size_t)PS2*PS2*PS2;
    int rc = ensure_staging( s, chunk );
    if ( rc != GB_OK ) return rc;
@@ -796,7 +796,7 @@ int gb_fluid_solve_device( gb_fluid_solver *s, const void *flu_in, void *flu_out
    if ( is_ctu( s ) )
    {
       // the plane-streaming kernel needs no scratch
-      const bool fused = gb::ctu_hydro_fused( s->cfg, npg );
+      const bool fused = gb::ctu_hydro_fused( s->cfg, *prm, npg );
       const int chunk = fused ? 0 : ( npg < mhd_chunk( s ) ) ? npg : mhd_chunk( s );
       if ( chunk > 0 && ( rc = ensure_scratch( s, 0, chunk ) ) != GB_OK ) return rc;
       s->last = (cudaStream_t)stream;

@@ -103,7 +103,7 @@ EXPORTED = ["gb_fluid_create", "gb_fluid_destroy", "gb_fluid_solve_device", "gb_
             "gb_flux_fixup_device", "gb_fluid_solve_host_async", "gb_fluid_synchronize",
             "gb_ctu_mhd_solve_static", "gb_ctu_mhd_static_capacity", "gb_interpolate_device",
             "gb_assemble_windows_device", "gb_fluid_correct_unphysical_mhd_device", "gb_flux_fixup_mhd_device",
-            "gb_mhd_fixup_electric_device", "gb_fluid_set_launch", "gb_fluid_get_launch"]
+            "gb_mhd_fixup_electric_device", "gb_fluid_set_launch", "gb_fluid_get_launch", "gb_fluid_ctu_one_kernel"]
 
 _lib = None
 
@@ -137,6 +137,7 @@ def load_library(path: str | None = None):
     lib.gb_fluid_set_block_size.argtypes = [vp, i]
     lib.gb_fluid_get_block_size.argtypes = [vp, ip]
     lib.gb_fluid_set_mhd_chunk.argtypes = [vp, i]
+    lib.gb_fluid_ctu_one_kernel.argtypes = [ctypes.POINTER(_Config), ctypes.POINTER(_Params), i, ip]
     lib.gb_fluid_set_launch.argtypes = [vp, i, i, i]
     lib.gb_fluid_get_launch.argtypes = [vp, ip, ip, ip]
     d = ctypes.c_double
@@ -367,6 +368,14 @@ class FluidSolver:
 
     def set_mhd_chunk(self, npg):
         _check(self.lib.gb_fluid_set_mhd_chunk(self.h, int(npg)), "gb_fluid_set_mhd_chunk")
+
+    def ctu_one_kernel(self, npg, params: SolverParams):
+        """Whether a hydro CTU call of npg patch groups runs as one kernel (gb_fluid_ctu_one_kernel)."""
+        one = ctypes.c_int()
+        p = params.c(self)
+        _check(self.lib.gb_fluid_ctu_one_kernel(ctypes.byref(self.cfg), ctypes.byref(p), int(npg), ctypes.byref(one)),
+               "gb_fluid_ctu_one_kernel")
+        return bool(one.value)
 
     def solve_device(self, flu_in, flu_out, params: SolverParams, flux=None, de_out=None, pg_fail=None,
                      stream=None, mag_in=None, mag_out=None, ele=None):

@@ -133,8 +133,8 @@ int gb_fluid_destroy( gb_fluid_solver *s );
  * pg_fail (optional, int[npg]) receives 1 for each patch group still unphysical after the retries.
  * A patch group's result does not depend on the others of the call, with one exception: hydro CTU
  * (five variables, primitive limiting) runs as one kernel when the call has enough patch groups and as
- * several kernels otherwise, and the two may differ in the last bits.  npg and the configuration
- * decide, so that the host-array calls below give the bits of this call whatever their chunks; a batch
+ * several kernels otherwise, and the two may differ in the last bits.  npg, the configuration and the
+ * limiter decide (gb_fluid_ctu_one_kernel), so that the host-array calls below give the bits of this call whatever their chunks; a batch
  * split over calls of other sizes need not. */
 int gb_fluid_solve_device( gb_fluid_solver *s, const void *flu_in, void *flu_out,
                            const void *mag_in, void *mag_out, char *de_out,
@@ -222,6 +222,11 @@ int gb_fluid_get_launch( gb_fluid_solver *s, int *threads, int *ctas_per_sm, int
  * is that of the copies.  Concurrent calls on one solver share the
  * scratch of the device entry point and must not overlap. */
 int gb_fluid_set_mhd_chunk( gb_fluid_solver *s, int npg );
+
+/* Whether a hydro CTU call of npg patch groups runs as one kernel on the current device (*one = 1) or as
+ * several (0); calls of the same answer give a patch group the same bits.  Of prm, the limiter and its
+ * coefficient are used. */
+int gb_fluid_ctu_one_kernel( const gb_fluid_config *cfg, const gb_fluid_params *prm, int npg, int *one );
 
 /* CTU + MHD solve that allocates no memory (no counterpart in the reference).  It is for callers
  * that cannot call cudaMalloc: a host code whose device memory is all owned by its own pool

@@ -171,3 +171,32 @@ def test_device_wrappers_reject_mismatched_arrays_before_any_launch():
     with pytest.raises(ValueError, match="flux"):
         s.flux_fixup_device(torch.zeros((3, 5, 8, 8, 8)), torch.zeros((3, 6, 6, 8, 8)),
                             torch.zeros((3, 6), dtype=torch.uint8), p)
+
+
+def test_ctu_kernel_rule_reaches_what_is_built(lib):
+    """Every configuration the plane-streaming CTU kernel is built for is chosen for some number of
+    patch groups, whole waves among them, and no other configuration ever is."""
+    plm, ppm = [("fp32", "plm"), ("mixed", "plm"), ("fp64", "plm")], [("fp32", "ppm")]
+    built = {c + (rs, "gminmod", 1.5) for c in plm + ppm for rs in ("hllc", "hlle")}
+    built |= {c + (rs, lim, th) for c in (plm[0], plm[2]) for rs in ("hllc", "hlle") for lim, th in (("vanleer", 1.5), ("gminmod", 2.0))}
+    built |= {ppm[0] + ("hllc", lim, th) for lim, th in (("vanleer", 1.5), ("gminmod", 2.0))}
+    one = ctypes.c_int(-1)
+    for prec in fluid.PRECISION:
+        for lr in fluid.LR:
+            for rs in ("exact", "roe", "hlle", "hllc", "hlld"):
+                for lim, theta in (("gminmod", 1.5), ("gminmod", 2.0), ("vanleer", 1.5)):
+                    prm = fluid.SolverParams(dt=1e-3, dh=1e-2, LR_Limiter=lim, MinMod_Coeff=theta).c()
+                    for de, char, npas in ((0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 2)):
+                        cfg = fluid._Config(fluid.SCHEME["ctu"], fluid.LR[lr], fluid.RSOLVER[rs], fluid.PRECISION[prec], de,
+                                            22 if lr == "ppm" else 20, 5 / 3, char, npas)
+                        hit = set()
+                        for n in range(0, 900):
+                            assert lib.gb_fluid_ctu_one_kernel(ctypes.byref(cfg), ctypes.byref(prm), n, ctypes.byref(one)) == 0
+                            if one.value:
+                                hit.add(n)
+                        if (prec, lr, rs, lim, theta) in built and not (de or char or npas):
+                            slots = 296 if lr == "plm" and prec != "fp64" else 148
+                            assert {k * slots for k in range(1, 899 // slots + 1)} <= hit and min(hit) > 60
+                        else:
+                            assert not hit
+    assert lib.gb_fluid_ctu_one_kernel(None, ctypes.byref(prm), 1, ctypes.byref(one)) == -1
