@@ -133,13 +133,14 @@ __global__ void __launch_bounds__( DT_BLOCK ) dt_cfl_kernel( const R *flu, const
 // the eight patches of one patch group of hydro solver outputs per CTA: each thread reads four
 // neighbouring cells of a variable with one 16-byte load, 64 threads a plane, so that a warp's rows
 // are whole 64-byte lines instead of the 32-byte halves of one patch.  Bound by DRAM (2048 patch groups,
-// FP32: 40.5 -> 36 us, the output alone 26 us).
+// FP32, after the fix-up: 40.5 -> 36 us, the output alone 26 us).
 constexpr int DT_PG_BLOCK = 256;
-// fewer than two such CTAs per SM leave it idle, and one CTA per patch is faster: a closing pass of a few
-// FP64 patch groups (correction, flux fix-up, dt) took 39.0 us by patches, 41.6 by patch groups
-// (444 patch groups, FP32: 16.3 -> 14.4 us).  FP64 reads whole lines either way: 600 patch groups 29.5 us by
-// patches, 32.7 by patch groups, so it stays with the patches
-constexpr int DT_PG_MIN = 296;
+// Patch groups per two SMs from which it is used: fewer CTAs leave SMs idle or in an uneven last round, and
+// one CTA per patch is faster.  us, by patches / by patch groups: FP32 300 patch groups 5.0 / 5.1, 350: 5.7 / 5.5,
+// 1000: 12.7 / 9.8; mixed, whose pressures are formed in double, 300: 6.5 / 8.2, 600: 10.5 / 12.0, 800: 13.6 / 13.7,
+// 1000: 18.2 / 15.8.  FP64 reads whole lines either way: 600 patch groups after the fix-up 29.5 / 32.7, so it stays
+// with the patches
+template <int P> constexpr int dt_pg_min() { return P == P_FP32 ? 5 : 12; }
 
 template <int P>
 __global__ void __launch_bounds__( DT_PG_BLOCK ) dt_cfl_pg_kernel( const float *flu, float *dt, int ncomp, Phys<float> ph, float dh_safety )
@@ -197,7 +198,10 @@ int launch_dt( const gb_fluid_config &c, const void *flu, const void *mag, void 
    const R dh_safety = (R)safety*(R)dh;
    if constexpr ( std::is_same<R,float>::value )
    {
-      if ( !cfg_mhd( c ) && from_output && npatch >= 8*DT_PG_MIN && ( (uintptr_t)flu & 15u ) == 0 )
+      int dev = 0, nsm = 148;
+      cudaGetDevice( &dev );
+      cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
+      if ( !cfg_mhd( c ) && from_output && npatch >= 4*dt_pg_min<P>()*nsm && ( (uintptr_t)flu & 15u ) == 0 )
       {
          dt_cfl_pg_kernel<P><<< npatch/8, DT_PG_BLOCK, 0, st >>>( (const float*)flu, (float*)dt, ncomp, ph, dh_safety );
          return ( cudaGetLastError() == cudaSuccess ) ? GB_OK : GB_E_CUDA;
