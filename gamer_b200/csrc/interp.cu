@@ -693,8 +693,11 @@ int assemble_launch( const void *fine, const int *nbr, const void *cint, void *w
 {
    const long long items = (long long)npg*ncomp;
    // few windows: several CTAs each, about four per SM in all
+   int dev = 0, nsm = 148;
+   cudaGetDevice( &dev );
+   cudaDeviceGetAttribute( &nsm, cudaDevAttrMultiProcessorCount, dev );
    const dim3 grid( (unsigned)( ( items < 0x7fffffffLL ) ? items : 0x7fffffffLL ),
-                    (unsigned)( ( items >= 592 ) ? 1 : ( items <= 74 ) ? 8 : 592/items ) );
+                    (unsigned)( ( items >= 4*nsm ) ? 1 : ( 2*items <= nsm ) ? 8 : 4*nsm/items ) );
    const bool vec = ( (uintptr_t)win & 15u ) == 0;
    const bool pair = ( ( (uintptr_t)fine | (uintptr_t)cint ) & ( 2*sizeof(R) - 1 ) ) == 0;
 #  define GB_ASM( N, V, P ) assemble_windows_kernel<R,N,V,P><<< grid, ASM_THREADS, 0, st >>>( (const R*)fine, nbr, (const R*)cint, (R*)win, npg, ncomp, nxt )
