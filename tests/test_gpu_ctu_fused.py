@@ -81,7 +81,7 @@ def test_streaming_kernel_without_flux_planes(cuda_device):
 @pytest.mark.parametrize("prec,lr,rs", [("fp32", "plm", "hllc"), ("mixed", "plm", "hllc"), ("fp32", "ppm", "hllc"), ("fp64", "plm", "hllc"),
                                         ("fp32", "plm", "hlle")])
 def test_streaming_kernel_rescues_faces_without_pressure(cuda_device, prec, lr, rs):
-    """Converging streams without pressure along x, y and z in some patch groups: the HLLC flux of their
+    """Streams without pressure along x, y and z in some patch groups: the HLLC flux of their
     faces is 0/0 and the HLLE flux stands in, in half and full step, for the x and the y lane of the packed
     solver each on its own.  Same as the separate kernels, whose solver is scalar."""
     import torch

@@ -135,3 +135,37 @@ def test_dt_of_an_aligned_array_is_not_slower(cuda_device, prec, npg):
     # 10 % for the spread of such short kernels; with the line at 296 patch groups in every policy mixed
     # took 1.27 and 1.14 times as long at 300 and 600
     assert us[0] < 1.1 * us[1], us
+
+
+@pytest.mark.parametrize("npgs", [(3, 5), (40, 0, 200, 61), (290, 37), (1, 296, 300)])
+@pytest.mark.parametrize("kw", [dict(precision="fp32"), dict(precision="mixed", dual_energy=True), dict(precision="fp64")])
+def test_slabs_of_a_multi_level_call(cuda_device, npgs, kw):
+    """Levels with time steps and cell sizes of their own, the slabs of the last wave across their
+    borders: the bits of the call that keeps its patch groups whole, and of one call per level."""
+    import torch
+    s = FluidSolver(gamma=GAMMA, **kw)
+    n = sum(npgs)
+    x, dt, dh = _windows(n, 20, s.np_dtype, s.dual)
+    t = torch.from_numpy(x).cuda()
+    dts, dhs = [dt / 2 ** l for l in range(len(npgs))], [dh / 2 ** l for l in range(len(npgs))]
+    got = []
+    for way in ("whole", "slabs", "levels"):
+        out = torch.full((n, s.ncomp, 16, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        flux = torch.full((n, 9, s.ncomp, 16, 16), float("nan"), dtype=t.dtype, device="cuda")
+        de = torch.full((n, 16, 16, 16), 48, dtype=torch.int8, device="cuda") if s.dual else None
+        if way == "levels":
+            a = 0
+            for m, d, h in zip(npgs, dts, dhs):
+                if m:
+                    s.solve_device(t[a:a + m], out[a:a + m], SolverParams(dt=d, dh=h), flux=flux[a:a + m],
+                                   de_out=None if de is None else de[a:a + m])
+                a += m
+        else:
+            s.solve_levels_device(t, out, npgs, dts, dhs, SolverParams(dt=dt, dh=dh), flux=flux, de_out=de,
+                                  pg_fail=torch.zeros(n, dtype=torch.int32, device="cuda") if way == "whole" else None)
+        torch.cuda.synchronize()
+        got.append((out, flux, de))
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert a is None or torch.equal(a, b)
+    assert bool(torch.isfinite(got[0][0]).all())
