@@ -330,9 +330,9 @@ GB_DEV bool child_fails( const IntArgs<R> &a, const R (&u)[5], bool prim )
 // over the variables they went through local memory.  Bound by the issue of the 19 one-dimensional
 // operators of a parent's variable, each of rounded multiplications and selects.
 // cquad, FP32, us, against one thread per parent of the whole call that makes all its attempts from
-// global memory: 342 regions of 12^3 cells 97 -> 62, with half of the parents iterating 233 -> 131; 4096:
-// 1196 -> 695 and 2810 -> 1250; 8000 regions of 4^3 cells 25.4 -> 18.1 (with a CTA per region 252); one
-// of 70^3 87.5 -> 88.7; a call of a few thousand parents, which is latency, 10.1 -> 10.9.
+// global memory: 342 regions of 12^3 cells 97 -> 54, with half of the parents iterating 233 -> 123; 4096:
+// 1196 -> 565 and 2810 -> 1380; 8000 regions of 4^3 cells 25.4 -> 16.6 (with a CTA per region 251); one
+// of 70^3 87.5 -> 80 (with a CTA per plane 172); a call of a few thousand parents, which is latency, 10.1 -> 10.2.
 constexpr int INT_THREADS = 256;
 
 // CTAs per SM: 342 regions of 12^3 cells, with the window assembly, us: FP32 1: 137, 2: 111, 3: 97, 4: 103
@@ -347,6 +347,53 @@ struct IntTile {
    int threads;
 };
 
+// one attempt of Interpolate_Iterate at the parent src[0] (variables vs apart), with its children stored at fo; false:
+// a child came out unphysical and another attempt may follow.  LATER: an attempt after the first, in
+// primitive variables if prim
+template <int SCH, bool LATER, typename R>
+GB_DEV bool int_attempt( const IntArgs<R> &a, const R *src, int sx, int sxy, int vs, R coeff, bool prim, bool more, R *fo, size_t fx,
+                         size_t fxy, size_t f3 )
+{
+   R f[5][2][2][2];
+#  pragma unroll
+   for (int v=0; v<5; v++)
+   {
+      children<SCH>( a, src + v*vs, sx, sxy, v, coeff, f[v] );
+      asm volatile( "" ::: "memory" );      // one variable's stencil live at a time
+   }
+   bool ok = true;
+#  pragma unroll
+   for (int q=0; q<8; q++)
+   {
+      R u[5];
+#     pragma unroll
+      for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+      ok &= !child_fails( a, u, LATER && prim );
+   }
+   if ( !ok && more ) return false;
+   if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
+   if ( LATER && prim )
+   {
+      // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
+#     pragma unroll
+      for (int q=0; q<8; q++)
+      {
+         const int z = q >> 2, y = ( q >> 1 ) & 1, x = q & 1;
+         const R d = f[0][z][y][x];
+         const R mx = rmul( d, f[1][z][y][x] ), my = rmul( d, f[2][z][y][x] ), mz = rmul( d, f[3][z][y][x] );
+         const R eint = rmul( f[4][z][y][x], a.inv_gm1 );
+         f[1][z][y][x] = mx;  f[2][z][y][x] = my;  f[3][z][y][x] = mz;
+         f[4][z][y][x] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( mx, mx ), rmul( my, my ) ), rmul( mz, mz ) ) ), d ), eint );
+      }
+   }
+   // (the two children along x, which share a sector, one after the other)
+#  pragma unroll
+   for (int v=0; v<5; v++)
+#     pragma unroll
+      for (int q=0; q<8; q++) fo[v*f3 + ( q >> 2 )*fxy + ( ( q >> 1 ) & 1 )*fx + ( q & 1 )] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
+   return true;
+}
+
 template <int SCH, typename R>
 __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_kernel( const __grid_constant__ IntArgs<R> a,
                                                                                         const __grid_constant__ IntTile w )
@@ -356,11 +403,12 @@ __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_k
    __shared__ int s_nfail[2];
    R *s_c = (R*)int_smem;
    const int tid = threadIdx.x, nth = blockDim.x;
-   const int nbox = w.nbox[0]*w.nbox[1]*w.nbox[2], box = blockIdx.x % nbox;
-   const int b0 = ( blockIdx.x / nbox )*w.m, nreg = ( a.nbatch - b0 < w.m ) ? a.nbatch - b0 : w.m;
-   // the box's first parent, its parents and its staged cells along each axis
-   const int o[3] = { ( box % w.nbox[0] )*w.n[0], ( box / w.nbox[0] % w.nbox[1] )*w.n[1], ( box / ( w.nbox[0]*w.nbox[1] ) )*w.n[2] };
-   int p[3];
+   // the region (the first of m) and the box of parents in it: its first parent and its extents
+   int o[3] = { 0, 0, 0 }, p[3], bi = blockIdx.x;
+   if ( w.nbox[0] > 1 ) { o[0] = ( bi % w.nbox[0] )*w.n[0];  bi /= w.nbox[0]; }
+   if ( w.nbox[1] > 1 ) { o[1] = ( bi % w.nbox[1] )*w.n[1];  bi /= w.nbox[1]; }
+   if ( w.nbox[2] > 1 ) { o[2] = ( bi % w.nbox[2] )*w.n[2];  bi /= w.nbox[2]; }
+   const int b0 = bi*w.m, nreg = ( a.nbatch - b0 < w.m ) ? a.nbatch - b0 : w.m;
 #  pragma unroll
    for (int d=0; d<3; d++) p[d] = ( a.crange[d] - o[d] < w.n[d] ) ? a.crange[d] - o[d] : w.n[d];
    const int sx = w.b[0], sxy = w.b[0]*w.b[1];
@@ -368,24 +416,30 @@ __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_k
    const size_t c3 = (size_t)cxy*a.csize[2];
    const int gx = a.cstart[0] + o[0] - G, gy = a.cstart[1] + o[1] - G, gz = a.cstart[2] + o[2] - G;
    if ( tid < 2 ) s_nfail[tid] = 0;
-   if ( sx == cx && w.b[1] == a.csize[1] )
+   if ( sx == cx && w.b[1] == a.csize[1] && ( w.m == 1 || w.b[2] == a.csize[2] ) )
    {
-      // whole planes: one run per variable, or one in all for whole regions; 16-byte loads where every run
-      // starts on a 16-byte boundary
+      // whole planes, one run per variable (one in all for several regions, which are whole); 16-byte loads
+      // where every run starts on a 16-byte boundary
       constexpr int V = 16/sizeof(R);
-      const bool whole = ( w.b[2] == a.csize[2] );
-      const int nrun = whole ? 1 : 5*nreg, len = whole ? nreg*5*w.cells : ( p[2] + 2*G )*cxy;
-      const size_t first = (size_t)b0*5*c3 + (size_t)gz*cxy;
-      const bool vec = ( (uintptr_t)( a.cdata + first ) & 15u ) == 0 && ( nrun == 1 || ( c3 % V == 0 && w.cells % V == 0 ) );
-      for (int r=0; r<nrun; r++)
+      const R *src = a.cdata + (size_t)b0*5*c3 + (size_t)gz*cxy;
+      const bool aligned = ( (uintptr_t)src & 15u ) == 0;
+      if ( w.m == 1 )
       {
-         const R *src = a.cdata + first + r*c3;
-         R *dst = s_c + r*w.cells;
-         const int nv = vec ? len/V : 0;
-#        pragma unroll 4
-         for (int e = tid; e < nv; e += nth) ( (uint4*)dst )[e] = ( (const uint4*)src )[e];
-#        pragma unroll 4
-         for (int e = nv*V + tid; e < len; e += nth) dst[e] = src[e];
+         const int len = ( p[2] + 2*G )*cxy, nv = ( aligned && c3 % V == 0 && w.cells % V == 0 ) ? len/V : 0;
+         for (int e = tid; e < nv; e += nth)
+#           pragma unroll
+            for (int v=0; v<5; v++) ( (uint4*)( s_c + v*w.cells ) )[e] = ( (const uint4*)( src + v*c3 ) )[e];
+         for (int e = nv*V + tid; e < len; e += nth)
+#           pragma unroll
+            for (int v=0; v<5; v++) s_c[v*w.cells + e] = src[v*c3 + e];
+      }
+      else
+      {
+         const int len = nreg*5*w.cells, nv = aligned ? len/V : 0;
+#        pragma unroll 8
+         for (int e = tid; e < nv; e += nth) ( (uint4*)s_c )[e] = ( (const uint4*)src )[e];
+#        pragma unroll 8
+         for (int e = nv*V + tid; e < len; e += nth) s_c[e] = src[e];
       }
    }
    else
@@ -406,63 +460,46 @@ __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_k
    const int np = p[0]*p[1]*p[2], mono_iter = a.mono_max_iter, max_iter = a.int_prim ? mono_iter + 1 : mono_iter;
    unsigned short *list = (unsigned short*)( int_smem + w.list );        // [2][the CTA's parents]
    const int nlist = w.m*w.n[0]*w.n[1]*w.n[2];
-   R coeff = a.mono_coeff;
-   bool prim = false;
-   int n = nreg*np;
-   for (int it=0; ; it++)
+   // Interpolate_Iterate stores from the origin of the fine region
+   R *const f0 = a.fdata + (size_t)b0*5*f3 + (size_t)( 2*o[2] )*fxy + (size_t)( 2*o[1] )*fx + 2*o[0];
+   // parent id of the CTA: its staged cell and its first child
+   auto parent = [&]( int id, const R *&src, R *&fo )
    {
-      const unsigned short *cur = list + ( it & 1 )*nlist;
-      unsigned short *next = list + ( ( it + 1 ) & 1 )*nlist;
-      for (int e = tid; e < n; e += nth)
+      unsigned c = id, kk, jj;
+      src = s_c + G*( sxy + sx + 1 );
+      fo = f0;
+      if ( w.m > 1 )
       {
-         const int id = ( it == 0 ) ? e : cur[e];
-         const int r = id / np, c = id - r*np;
-         const int ii = c % p[0], jj = c / p[0] % p[1], kk = c / ( p[0]*p[1] );
-         const R *src = s_c + r*5*w.cells + ( kk + G )*sxy + ( jj + G )*sx + ii + G;
-         R f[5][2][2][2];
-#        pragma unroll
-         for (int v=0; v<5; v++)
-         {
-            children<SCH>( a, src + v*w.cells, sx, sxy, v, coeff, f[v] );
-            asm volatile( "" ::: "memory" );      // one variable's stencil live at a time
-         }
-         bool ok = true;
-#        pragma unroll
-         for (int q=0; q<8; q++)
-         {
-            R u[5];
-#           pragma unroll
-            for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
-            ok &= !child_fails( a, u, prim );
-         }
-         if ( !ok && it < max_iter ) { next[atomicAdd( &s_nfail[it & 1], 1 )] = (unsigned short)id;  continue; }
-         if ( !ok ) atomicOr( a.status, GB_INTERP_FAILED );
-         // Interpolate_Iterate stores from the origin of the fine region
-         R *fo = a.fdata + (size_t)( b0 + r )*5*f3 + (size_t)( 2*( o[2] + kk ) )*fxy + (size_t)( 2*( o[1] + jj ) )*fx + 2*( o[0] + ii );
-#        pragma unroll
-         for (int q=0; q<8; q++)
-         {
-            R u[5];
-#           pragma unroll
-            for (int v=0; v<5; v++) u[v] = f[v][q >> 2][( q >> 1 ) & 1][q & 1];
-            if ( prim )
-            {
-               // Hydro_Pri2Con: momenta rho*v, E = 1/2 |m|^2/rho + P/(gamma-1) (Hydro_ConEint2Etot)
-               const R d = u[0];
-               u[1] = rmul( d, u[1] );  u[2] = rmul( d, u[2] );  u[3] = rmul( d, u[3] );
-               const R eint = rmul( u[4], a.inv_gm1 );
-               u[4] = radd( rdiv( rmul( R(0.5), radd( radd( rmul( u[1], u[1] ), rmul( u[2], u[2] ) ), rmul( u[3], u[3] ) ) ), d ), eint );
-            }
-#           pragma unroll
-            for (int v=0; v<5; v++) fo[v*f3 + ( q >> 2 )*fxy + ( ( q >> 1 ) & 1 )*fx + ( q & 1 )] = u[v];
-         }
+         const unsigned r = c / (unsigned)np;
+         c -= r*np;
+         src += r*5*w.cells;
+         fo += r*5*f3;
       }
-      if ( it == max_iter ) return;
+      jj = c / (unsigned)p[0];
+      c -= jj*p[0];
+      kk = jj / (unsigned)p[1];
+      jj -= kk*p[1];
+      src += kk*sxy + jj*sx + c;
+      fo += 2*( kk*fxy + jj*fx + c );
+   };
+   int n = nreg*np;
+   for (int id = tid; id < n; id += nth)
+   {
+      const R *src;
+      R *fo;
+      parent( id, src, fo );
+      if ( !int_attempt<SCH,false>( a, src, sx, sxy, w.cells, a.mono_coeff, false, max_iter > 0, fo, fx, fxy, f3 ) )
+         list[atomicAdd( &s_nfail[0], 1 )] = (unsigned short)id;
+   }
+   if ( max_iter == 0 ) return;
+   R coeff = a.mono_coeff;
+   for (int it=1; ; it++)
+   {
       __syncthreads();
-      n = s_nfail[it & 1];
+      n = s_nfail[( it + 1 ) & 1];
       if ( n == 0 ) return;
-      if ( tid == 0 ) s_nfail[( it + 1 ) & 1] = 0;
-      if ( it == 0 && a.int_prim )
+      if ( tid == 0 ) s_nfail[it & 1] = 0;
+      if ( it == 1 && a.int_prim )
       {
          for (int e = tid; e < nreg*w.cells; e += nth)
          {
@@ -473,16 +510,26 @@ __global__ void __launch_bounds__( INT_THREADS, int_ctas<R>() ) interp_iterate_k
 #           pragma unroll
             for (int v=0; v<5; v++) q[v*w.cells] = u[v];
          }
-         prim = true;
       }
       else coeff = rmax( rsub( coeff, rdiv( a.mono_coeff, (R)mono_iter ) ), R(0) );
       __syncthreads();
+      const unsigned short *cur = list + ( ( it + 1 ) & 1 )*nlist;
+      unsigned short *next = list + ( it & 1 )*nlist;
+      for (int e = tid; e < n; e += nth)
+      {
+         const R *src;
+         R *fo;
+         parent( cur[e], src, fo );
+         if ( !int_attempt<SCH,true>( a, src, sx, sxy, w.cells, coeff, a.int_prim != 0, it < max_iter, fo, fx, fxy, f3 ) )
+            next[atomicAdd( &s_nfail[it & 1], 1 )] = cur[e];
+      }
+      if ( it == max_iter ) return;
    }
 }
 
 // The boxes of a call.  A round of 256 parents on an SM that holds a full set of CTAs takes one unit of
-// time, alone on its SM `alone` units (measured for 12^3 regions: 8.3 and 11.7 us in FP32, 15 us both
-// in FP64), the staging of 256 cells 0.06 (of a cell by one thread 0.03) and the launch of a CTA 0.05; the choice is the one for which the slowest SM, or the
+// time, alone on its SM `alone` units (measured for 12^3 regions: 8.3 and 11.7 us in FP32, 15 us both in
+// FP64), the staging of 256 cells 0.06 (of a cell by one thread 0.03) and the launch of a CTA 0.05; the choice is the one for which the slowest SM, or the
 // chain of rounds of the CTAs that follow each other in one place, takes least, and the largest box
 // of those that tie.  At most 48 KB of shared memory.
 template <typename R>
@@ -508,9 +555,9 @@ IntTile interp_tile( int scheme, const IntArgs<R> &a, int nsm )
       for (int d=0; d<3; d++) { t.nbox[d] = ( a.crange[d] + t.n[d] - 1 )/t.n[d];  t.b[d] = t.n[d] + 2*G; }
       t.cells = (int)cells;
       t.list  = (int)list;
-      const int warps = ( parents >= INT_THREADS ) ? INT_THREADS/32 : (int)( parents + 31 )/32;
+      const int rounds = (int)( ( parents + INT_THREADS - 1 )/INT_THREADS );
+      const int warps = (int)( ( parents + 32*rounds - 1 )/( 32*rounds ) );
       t.threads = 32*warps;
-      const int rounds = (int)( ( parents + t.threads - 1 )/t.threads );
       // CTAs that share an SM: by registers and by shared memory
       int share = int_ctas<R>()*( INT_THREADS/32 )/warps;
       const int fit = 227*1024/( t.list + 4*(int)parents + 1024 );
@@ -549,7 +596,7 @@ IntTile interp_tile( int scheme, const IntArgs<R> &a, int nsm )
          if ( last != 1 ) fits |= consider( 1, px, py, 1 );
          if ( py == 1 || ( fits && (long long)a.nbatch*ky*nz >= 2*nsm ) ) break;
       }
-      if ( px == 1 || ( fits && ( px < 32 || best.threads == INT_THREADS || region*a.nbatch < (long long)nsm*INT_THREADS ) ) ) return best;
+      if ( px == 1 || ( fits && ( px < 32 || best.threads >= INT_THREADS/2 || region*a.nbatch < (long long)nsm*INT_THREADS ) ) ) return best;
    }
 }
 
