@@ -1085,8 +1085,12 @@ def main():
         x, dt, dh = make_inputs(nxt)
         npg_full = x.shape[0]
         # every step is the whole workload (all patch groups), as in this solver's arm
-        v, t = run_reference_cpu(x, dt, dh, variant, "fp64" if args.precision == "fp64" else "fp32",
-                                 args.steps, args.warmup, npg_full, threads)
+        try:
+            v, t = run_reference_cpu(x, dt, dh, variant, "fp64" if args.precision == "fp64" else "fp32",
+                                     args.steps, args.warmup, npg_full, threads)
+        except FileNotFoundError as e:
+            print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+            return 0
         line = {"impl": "reference", "metric": headline_metric(args),
                 "value": v, "unit": "cell-updates/s", "n_gpus": args.gpus, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": t * 1e3, "higher_is_better": True,

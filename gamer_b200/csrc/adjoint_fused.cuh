@@ -15,9 +15,10 @@
 // Sums are in double as in the separate kernels.  The planes of the input (ring of 5) and of
 // d loss / d U_out (ring of 4) arrive by 1-D bulk copies; 213 KB of shared memory, one CTA of 384
 // threads per SM at 162 registers.  The global traffic per patch group is the input, d loss / d U_out and
-// d loss / d U_in, 0.5 MB.  Bound by the issue of the double arithmetic, which is what a wave costs
-// whatever it holds: a wave of 148 patch groups takes 0.227 ms where the separate kernels take 0.33;
-// 1024 patch groups, two steps forward and back: 2.28 -> 1.71 ms a step.
+// d loss / d U_in, 0.5 MB.  Bound by the barriers between the phases and by dependent instructions, with three
+// warps per scheduler to hide them (42% of the issue slots), which is what a wave costs whatever it
+// holds: a wave of 148 patch groups takes 0.227 ms where the separate kernels take 0.33; 1024 patch
+// groups, two steps forward and back: 2.28 -> 1.71 ms a step.
 #pragma once
 #include "adjoint.cuh"
 #include "hydro_pair.cuh"

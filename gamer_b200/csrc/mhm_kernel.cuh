@@ -225,7 +225,9 @@ constexpr int RP_NX = 22, RP_NV = 20;
 
 // Registers: the float kernels are held to 96 per thread, so that two CTAs of 320 threads (the
 // default launch) share an SM; FP64 (one CTA of up to 384 per SM: three warps on each quarter) may use 168.
-// FP64 PLM, 512 patch groups: 255 registers and 256 threads 526 us, 168 and 384: 398, 352: 395.  REG != 0 caps them at
+// FP64 PLM, 512 patch groups: 255 registers and 256 threads 526 us, 168 and 384: 398, 352: 395.  Most FP64
+// instantiations spill at 168, and all gain: every solver, limiter kind, dual energy and user scalars, three
+// whole waves, 1.09 (Roe, characteristic limiting, 8 variables) to 1.7 times (PPM).  REG != 0 caps them at
 // REG instead (the autotuner's register variants: 64 / 72 / 80 let two CTAs of 512 / 448 / 384
 // threads share an SM, 128 two CTAs of 256).
 constexpr int mhm_maxnreg( int rsize, int reg ) { return reg ? reg : ( rsize == 8 ? 168 : 96 ); }

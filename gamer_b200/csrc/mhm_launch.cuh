@@ -12,7 +12,7 @@ using MhmLaunchFn = cudaError_t (*)( const MhmArgs<R> &, int block, int ctas_per
 // in slabs along z.  A slab of m output planes sweeps m + 2 G input planes, so the number of slabs is
 // the one for which the rest takes the fewest plane steps.  A patch group that may be retried with a
 // smaller MinMod coefficient, or whose failure is reported, stays whole: all of it is recomputed.
-// Measured on B200, us, whole patch groups -> with slabs: FP32 PLM HLLC 8 patch groups 63.6 -> 18.0,
+// Measured on B200, us, whole patch groups -> with slabs: FP32 PLM HLLC 8 patch groups 61.5 -> 12.5,
 // 64: 63.4 -> 30.4, 350: 139 -> 112 (200, of which each already has a slot: no slabs, 86);
 // PPM Roe mixed 1000: 692 -> 627; FP64 PLM 30: 149 -> 49, 512: 593 -> 526.
 template <typename R>

@@ -206,7 +206,7 @@ int gb_fluid_get_block_size( gb_fluid_solver *s, int *threads );
  *    threads        threads per CTA (0 = the tuned default; else as gb_fluid_set_block_size)
  *    ctas_per_sm    at most this many CTAs per SM in the persistent grid (0 = as many as fit; 1-8)
  *    max_registers  the register-capped instantiation of the kernel: 0 (default: 96 per thread in
- *                   float, 255 in FP64), 64, 72, 80 or 128; built for the float policies' MHM +
+ *                   float, 168 in FP64), 64, 72, 80 or 128; built for the float policies' MHM +
  *                   PLM + HLLC, 5 variables, FLU_NXT = 20, generalized MinMod (the headline
  *                   kernel); launches of other configurations use their default instantiation
  * Invalid values → GB_E_INVALID; a launch whose shape does not fit an SM fails with GB_E_CUDA. */
