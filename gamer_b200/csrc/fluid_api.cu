@@ -348,12 +348,15 @@ int ensure_staging( gb_fluid_solver *s, size_t npg )
 int solve_host_ctu( gb_fluid_solver *s, const void *flu_in, void *flu_out, const void *mag_in, void *mag_out,
                     void *flux, void *ele, char *de_out, int npg, const gb_fluid_params *prm )
 {
-   int chunk = ( mhd_chunk( s ) < GB_HOST_CTU_CHUNK ) ? mhd_chunk( s ) : GB_HOST_CTU_CHUNK;
-   if ( npg < chunk ) chunk = npg;
-   const bool dual = ( s->cfg.dual_energy == GB_DE_ENPY );
    // the kernel is chosen by the patch groups of the whole call, so that every chunk rounds alike (and like
    // the same call on device arrays); the plane-streaming one needs no scratch
    const bool fused = !is_mhd( s ) && gb::ctu_hydro_fused( s->cfg, *prm, npg );
+   int chunk = ( mhd_chunk( s ) < GB_HOST_CTU_CHUNK ) ? mhd_chunk( s ) : GB_HOST_CTU_CHUNK;
+   // a launch of it takes the time of a wave however few its patch groups: the copies of 64 hide it (FP32,
+   // 560 patch groups, 16: 3160 us, 64: 2330; the separate kernels in chunks of 16: 2590, of 64: 2220)
+   if ( fused && chunk < 64 ) chunk = 64;
+   if ( npg < chunk ) chunk = npg;
+   const bool dual = ( s->cfg.dual_energy == GB_DE_ENPY );
    const size_t bd = (size_t)PS2*PS2*PS2;
    int rc = ensure_staging( s, chunk );
    if ( rc != GB_OK ) return rc;

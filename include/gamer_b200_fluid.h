@@ -219,7 +219,7 @@ int gb_fluid_get_launch( gb_fluid_solver *s, int *threads, int *ctas_per_sm, int
  * FP64) per patch group of the largest chunk used so far (a call of fewer patch groups than the
  * chunk needs only those), allocated on first use.  The hydro calls that run as one kernel (see
  * gb_fluid_solve_device) use no scratch: on device arrays they are not chunked, on host arrays the chunk
- * is that of the copies.  Concurrent calls on one solver share the
+ * is that of the copies, 64 at least.  Concurrent calls on one solver share the
  * scratch of the device entry point and must not overlap. */
 int gb_fluid_set_mhd_chunk( gb_fluid_solver *s, int npg );
 
